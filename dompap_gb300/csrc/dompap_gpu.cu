@@ -3844,11 +3844,10 @@ struct dp_mlp {
     float *master = nullptr, *mo = nullptr, *ve = nullptr, *grad = nullptr, *norm = nullptr, *loss = nullptr;
     unsigned long long* gradfx = nullptr;  // DP_MLP_NPARAM + 1 (the loss last)
     dp_mlp_dev* dev = nullptr;
+    uint32_t* w2t = nullptr;  // bf16 fragments of W2 transposed (backward pass)
     float* s = nullptr;
     float2* t = nullptr;
     long long n = 0;
-    long long* idx = nullptr;
-    long long idx_cap = 0;
     float* losses = nullptr;
     long long losses_cap = 0;
     long long step = 0;
@@ -3856,34 +3855,50 @@ struct dp_mlp {
 };
 
 static int mlp_pack(dp_mlp* m) {
-    k_mlp_pack<<<4, 256, 0, m->stream>>>(m->master, m->norm, m->dev);
+    k_mlp_pack<<<4, 256, 0, m->stream>>>(m->master, m->norm, m->dev, m->w2t);
     CK(cudaGetLastError());
     return DP_OK;
 }
 
-static int mlp_grad_launch(dp_mlp* m, const float* s, const float2* t, const long long* idx, long long batch,
-                           float wf, bool accurate) {
+// Launch with programmatic dependent launch: the kernel's blocks may be placed
+// while the one before it on the stream still runs; both kernels of a training
+// step wait (griddepcontrol.wait) before they touch anything it writes.
+template <typename Args>
+static cudaError_t mlp_launch(void (*kernel)(Args), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                              const Args& args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
+static MlpTrainArgs mlp_grad_args(const dp_mlp* m, const float* s, const float2* t, long long batch, float wf) {
     MlpTrainArgs a;
+    memset(&a, 0, sizeof(a));
     a.s = s;
     a.t = t;
-    a.idx = idx;
     a.batch = batch;
     a.mdev = m->dev;
-    a.master = m->master;
+    a.w2t = m->w2t;
     a.gradfx = m->gradfx;
     a.lossfx = m->gradfx + DP_MLP_NPARAM;
     a.wf = wf;
     a.inv_batch = 1.0f / (float)batch;
-    CK(cudaMemsetAsync(m->gradfx, 0, (DP_MLP_NPARAM + 1) * sizeof(unsigned long long), m->stream));
-    const long long tiles = (batch + 15) / 16;
-    const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>((tiles + 7) / 8, 152LL * 4));
-    if (accurate)
-        k_mlp_grad<true><<<grid, 256, DP_MLP_GRAD_SMEM, m->stream>>>(a);
-    else
-        k_mlp_grad<false><<<grid, 256, DP_MLP_GRAD_SMEM, m->stream>>>(a);
-    k_mlp_grad_finish<<<grid_for(DP_MLP_NPARAM, kBlock), kBlock, 0, m->stream>>>(a.gradfx, a.lossfx, m->grad,
-                                                                                   m->loss);
-    CK(cudaGetLastError());
+    return a;
+}
+
+// Adds the batch's gradient and loss to gradfx (which the caller has cleared).
+static int mlp_grad_launch(dp_mlp* m, const MlpTrainArgs& a, bool accurate) {
+    const long long groups = (a.batch + DP_MLP_ROWS - 1) / DP_MLP_ROWS;
+    const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(groups, 152LL * 4));
+    CK(mlp_launch(accurate ? k_mlp_grad<true> : k_mlp_grad<false>, grid, 256, DP_MLP_GRAD_SMEM, m->stream, a));
     return DP_OK;
 }
 
@@ -3897,7 +3912,7 @@ int dp_mlp_create(dp_mlp** out) {
     if ((rc = dalloc_t(&m->master, DP_MLP_NPARAM)) || (rc = dalloc_t(&m->mo, DP_MLP_NPARAM)) ||
         (rc = dalloc_t(&m->ve, DP_MLP_NPARAM)) || (rc = dalloc_t(&m->grad, DP_MLP_NPARAM)) ||
         (rc = dalloc_t(&m->norm, 4)) || (rc = dalloc_t(&m->loss, 1)) || (rc = dalloc_t(&m->dev, 1)) ||
-        (rc = dalloc_t(&m->gradfx, DP_MLP_NPARAM + 1))) {
+        (rc = dalloc_t(&m->gradfx, DP_MLP_NPARAM + 1)) || (rc = dalloc_t(&m->w2t, 4 * 8 * 32 * 2))) {
         dp_mlp_destroy(m);
         return rc;
     }
@@ -3919,8 +3934,8 @@ int dp_mlp_create(dp_mlp** out) {
 int dp_mlp_destroy(dp_mlp* m) {
     if (!m) return DP_OK;
     if (m->stream) cudaStreamSynchronize(m->stream);
-    void* bufs[] = {m->master, m->mo, m->ve, m->grad, m->norm, m->loss, m->dev, m->s, m->t, m->idx, m->losses,
-                    m->gradfx};
+    void* bufs[] = {m->master, m->mo, m->ve, m->grad, m->norm, m->loss, m->dev, m->s, m->t, m->losses,
+                    m->gradfx, m->w2t};
     for (void* p : bufs)
         if (p) cudaFree(p);
     if (m->stream) cudaStreamDestroy(m->stream);
@@ -3971,28 +3986,30 @@ int dp_mlp_train(dp_mlp* m, int64_t steps, int batch, float lr0, float lr1, floa
                  float* losses) {
     if (!m || !m->s) return fail(DP_ERR_ARG, "no training data");
     if (steps < 1 || batch < 16) return fail(DP_ERR_ARG, "bad steps / batch");
-    if (batch > m->idx_cap) {
-        RET(dalloc_t(&m->idx, (size_t)batch));
-        m->idx_cap = batch;
-    }
     if (steps > m->losses_cap) {
         RET(dalloc_t(&m->losses, (size_t)steps));
         m->losses_cap = steps;
     }
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    MlpTrainArgs ga = mlp_grad_args(m, m->s, m->t, batch, wf);
+    ga.draw = 1;
+    ga.n = (unsigned long long)m->n;
+    ga.seed = seed;
+    MlpUpdateArgs ua = {m->master, m->mo, m->ve, ga.gradfx, ga.lossfx, m->dev, m->w2t, m->losses, 0.f, b1, b2, eps,
+                        0.f, 0.f};
+    // cleared once: k_mlp_update leaves the sums at zero
+    CK(cudaMemsetAsync(m->gradfx, 0, (DP_MLP_NPARAM + 1) * sizeof(unsigned long long), m->stream));
     for (long long k = 0; k < steps; ++k) {
         // cosine decay from lr0 to lr1
         const double frac = steps > 1 ? (double)k / (double)(steps - 1) : 1.0;
-        const float lr = (float)(lr1 + 0.5 * (lr0 - lr1) * (1.0 + std::cos(3.141592653589793 * frac)));
-        k_mlp_sample<<<grid_for(batch, kBlock), kBlock, 0, m->stream>>>(m->idx, batch, m->n, seed, m->step);
-        RET(mlp_grad_launch(m, m->s, m->t, m->idx, batch, wf, accurate != 0));
-        CK(cudaMemcpyAsync(m->losses + k, m->loss, sizeof(float), cudaMemcpyDeviceToDevice, m->stream));
+        ua.lr = (float)(lr1 + 0.5 * (lr0 - lr1) * (1.0 + std::cos(3.141592653589793 * frac)));
+        ga.step = m->step;
+        RET(mlp_grad_launch(m, ga, accurate != 0));
         ++m->step;
-        const float c1 = 1.0f / (1.0f - std::pow(b1, (float)m->step));
-        const float c2 = 1.0f / (1.0f - std::pow(b2, (float)m->step));
-        k_mlp_adam<<<grid_for(DP_MLP_NPARAM, kBlock), kBlock, 0, m->stream>>>(m->master, m->mo, m->ve, m->grad, lr,
-                                                                               b1, b2, eps, c1, c2);
-        RET(mlp_pack(m));
+        ua.c1 = 1.0f / (1.0f - std::pow(b1, (float)m->step));
+        ua.c2 = 1.0f / (1.0f - std::pow(b2, (float)m->step));
+        ua.loss = m->losses + k;
+        CK(mlp_launch(k_mlp_update, (kMlpUpdateThreads + 63) / 64, 64, 0, m->stream, ua));
     }
     CK(cudaGetLastError());
     if (losses) CK(cudaMemcpyAsync(losses, m->losses, (size_t)steps * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
@@ -4031,7 +4048,15 @@ int dp_mlp_gradients(dp_mlp* m, const float* s, const float* targets, int64_t n,
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(buf + toff, targets, (size_t)n * 2 * sizeof(float), cudaMemcpyHostToDevice, m->stream);
     int rc = DP_OK;
-    if (e == cudaSuccess) rc = mlp_grad_launch(m, buf, (const float2*)(buf + toff), nullptr, n, wf, accurate != 0);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(m->gradfx, 0, (DP_MLP_NPARAM + 1) * sizeof(unsigned long long), m->stream);
+    if (e == cudaSuccess)
+        rc = mlp_grad_launch(m, mlp_grad_args(m, buf, (const float2*)(buf + toff), n, wf), accurate != 0);
+    if (e == cudaSuccess && rc == DP_OK) {
+        k_mlp_grad_finish<<<grid_for(DP_MLP_NPARAM, kBlock), kBlock, 0, m->stream>>>(
+            m->gradfx, m->gradfx + DP_MLP_NPARAM, m->grad, m->loss);
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess && rc == DP_OK)
         e = cudaMemcpyAsync(grad, m->grad, DP_MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
     float l = 0.f;
