@@ -8,7 +8,12 @@ derived symbolically, and the three are printed as templated device functions
     template <typename R> __device__ R dp_pair_f(R r, R dp_inv_r);   // -du/dr
     template <typename R> __device__ R dp_pair_c(R r, R dp_inv_r);   // d2u/dr2
 
-that ``pair_kernels.cuh`` inlines into its neighbour loops (the cut ``r >
+and, where ``u`` has only even powers of ``r`` (Lennard-Jones and its kin),
+
+    #define DP_PAIR_EVEN 1
+    template <typename R> __device__ R dp_pair_g(R q, R dp_inv_q);   // -du/dr / r at q = r^2
+
+which needs no square root, that ``pair_kernels.cuh`` inlines into its neighbour loops (the cut ``r >
 r_cut -> 0`` is applied there). ``dp_inv_r`` is ``1/r``, which the kernels get
 from one reciprocal square root together with ``r``; negative integer powers
 of ``r`` are printed as powers of it, so they cost no division. ``R`` is
@@ -158,6 +163,30 @@ def _horner(expr: sp.Expr) -> sp.Expr:
     return sp.horner(sp.expand(expr), wrt=x)
 
 
+_Q, _INV_Q = sp.Symbol("q"), sp.Symbol("dp_inv_q")
+
+
+def _even_source(f: sp.Expr) -> str:
+    """dp_pair_g(q, 1/q) = f(r)/r at q = r^2 where that is a polynomial in q and
+    1/q, else an empty string."""
+    terms = []
+    for term in sp.Add.make_args(sp.expand(f / R_SYM)):
+        coefficient, power = term.as_coeff_exponent(R_SYM)
+        if coefficient.has(R_SYM) or not power.is_Integer or int(power) % 2 or not coefficient.is_number:
+            return ""
+        k = int(power) // 2
+        if abs(k) > 64:
+            return ""
+        terms.append(coefficient * (_Q**k if k >= 0 else _INV_Q ** (-k)))
+    expr = _horner(sp.Add(*terms))
+    printer = _CudaPrinter()
+    repl, reduced = sp.cse(expr, symbols=sp.numbered_symbols("dp_t"))
+    lines = ["#define DP_PAIR_EVEN 1",
+             "template <typename R> __device__ __forceinline__ R dp_pair_g(R q, R dp_inv_q) {"]
+    lines += [f"    const R {sym} = {printer.doprint(sub)};" for sym, sub in repl]
+    return "\n".join(lines + [f"    return {printer.doprint(reduced[0])};", "}"])
+
+
 def _function_source(name: str, expr: sp.Expr, shift_literal: str | None = None, horner: bool = False) -> str:
     printer = _CudaPrinter()
     expr, _ = _share_reciprocal(expr)
@@ -208,6 +237,7 @@ def make_pair_source(pair_potential_str: str, r_cut: float) -> tuple[str, float]
         _function_source("dp_pair_u", u, shift_literal=_hex(shift)),
         _function_source("dp_pair_f", f, horner=True),
         _function_source("dp_pair_c", c),
+        _even_source(f),
     ])
     return src, float(r_cut)
 

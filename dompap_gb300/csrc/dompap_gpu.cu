@@ -1372,7 +1372,8 @@ struct dp_sim {
     int ntypes = 1;
     double sigma = 1.0, epsilon = 1.0, sig_max = 1.0;
     double *sig_tab = nullptr, *eps_tab = nullptr, *isig_tab = nullptr;
-    float2* ff_tab = nullptr;  // (sigma, 1/sigma, epsilon) double-float triples per type pair
+    float2* ff_tab = nullptr;  // DP_FF_PARAMS double-floats per type pair (pair_consts)
+    float4* f32_tab = nullptr; // sigma, 1/sigma, epsilon per type pair
 
     // neighbour list
     double skin = 1.0;
@@ -1731,6 +1732,21 @@ static int launch_rebuild(dp_sim* s, long long* launches) {
     return DP_OK;
 }
 
+// The pair kernels' constants of one (sigma, epsilon): sigma, 1/sigma,
+// epsilon, 1/sigma^2, epsilon/sigma (DP_FF_PARAMS), as double-floats in the
+// parity mode and as float32 otherwise.
+static void pair_consts(double sigma, double epsilon, double* c) {
+    c[0] = sigma;
+    c[1] = 1.0 / sigma;
+    c[2] = epsilon;
+    c[3] = 1.0 / (sigma * sigma);
+    c[4] = epsilon / sigma;
+}
+static float2 split_ff(double v) { return make_float2((float)v, (float)(v - (double)(float)v)); }
+static float4 pair_consts_f32(const double* c) {
+    return make_float4((float)c[0], (float)c[1], (float)c[2], 0.0f);
+}
+
 static void fill_pair_args(const dp_sim* s, dp_pair_args& a, double* out) {
     memset(&a, 0, sizeof(a));
     a.pos = s->pos;
@@ -1742,6 +1758,7 @@ static void fill_pair_args(const dp_sim* s, dp_pair_args& a, double* out) {
     a.eps_tab = s->eps_tab;
     a.isig_tab = s->isig_tab;
     a.ff_tab = s->ff_tab;
+    a.f32_tab = s->f32_tab;
     a.pos64 = s->pos64;
     a.order = s->order;
     a.out = out;
@@ -1762,12 +1779,20 @@ static void fill_pair_args(const dp_sim* s, dp_pair_args& a, double* out) {
     a.rcut = s->r_cut;
     a.rcut_f = (float)s->r_cut;
     a.rcut_finite = std::isfinite(s->r_cut) ? 1 : 0;
+    a.rcut2_f = (float)(s->r_cut * s->r_cut);
     {
-        const double c3[3] = {a.sigma, a.inv_sigma, a.epsilon};
-        for (int t = 0; t < 3; ++t) {
-            a.ff_const[2 * t] = (float)c3[t];
-            a.ff_const[2 * t + 1] = (float)(c3[t] - (double)(float)c3[t]);
+        double c[DP_FF_PARAMS];
+        pair_consts(s->sigma, s->epsilon, c);
+        for (int t = 0; t < DP_FF_PARAMS; ++t) {
+            const float2 v = split_ff(c[t]);
+            a.ff_const[2 * t] = v.x;
+            a.ff_const[2 * t + 1] = v.y;
         }
+        const float4 f = pair_consts_f32(c);
+        a.f32_const[0] = f.x;
+        a.f32_const[1] = f.y;
+        a.f32_const[2] = f.z;
+        a.f32_const[3] = f.w;
     }
     // Pre-filter threshold: a pair is skipped only when its float32 distance,
     // whose error is < 1e-6 relative plus a few L / 2^32, certainly exceeds
@@ -2448,7 +2473,7 @@ int dp_destroy(dp_sim* s) {
     free_graphs(s);
     void* bufs[] = {s->pos, s->vel, s->beta, s->force, s->pos_ref, s->img, s->shadow, s->shadow_ref, s->pos64,
                     s->pos_alt, s->shadow_alt, s->pos64_alt, s->mlp_fx,
-                    s->ff_tab, s->bk_pos,
+                    s->ff_tab, s->f32_tab, s->bk_pos,
                     s->bk_vel, s->bk_beta, s->bk_img, s->mclass, s->mcoef, s->mcoef_f, s->class_mass_dev, s->mass, s->types,
                     s->sig_tab, s->eps_tab, s->isig_tab, s->nl, s->cnt, s->bin_cnt, s->bin_start, s->bin_part,
                     s->bin_key, s->bin_rank, s->src_of, s->order, s->slot_of, s->sc_vel, s->sc_beta, s->sc_mass,
@@ -2826,15 +2851,18 @@ int dp_set_pair_params(dp_sim* s, int mode, int ntypes, const double* sigma, con
         CK(cudaMemcpy(s->sig_tab, sigma, m * sizeof(double), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(s->eps_tab, epsilon, m * sizeof(double), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(s->isig_tab, inv.data(), m * sizeof(double), cudaMemcpyHostToDevice));
-        std::vector<float2> ff(3 * m);
-        auto split = [](double v) { return make_float2((float)v, (float)(v - (double)(float)v)); };
+        std::vector<float2> ff(DP_FF_PARAMS * m);
+        std::vector<float4> f32(m);
         for (size_t t = 0; t < m; ++t) {
-            ff[3 * t + 0] = split(sigma[t]);
-            ff[3 * t + 1] = split(inv[t]);
-            ff[3 * t + 2] = split(epsilon[t]);
+            double c[DP_FF_PARAMS];
+            pair_consts(sigma[t], epsilon[t], c);
+            for (int q = 0; q < DP_FF_PARAMS; ++q) ff[DP_FF_PARAMS * t + q] = split_ff(c[q]);
+            f32[t] = pair_consts_f32(c);
         }
         RET(dalloc_t(&s->ff_tab, ff.size()));
         CK(cudaMemcpy(s->ff_tab, ff.data(), ff.size() * sizeof(float2), cudaMemcpyHostToDevice));
+        RET(dalloc_t(&s->f32_tab, f32.size()));
+        CK(cudaMemcpy(s->f32_tab, f32.data(), f32.size() * sizeof(float4), cudaMemcpyHostToDevice));
         s->ntypes = ntypes;
     } else if (mode == DP_PAIR_DENSE) {
         const size_t m = (size_t)s->n * s->n;

@@ -15,6 +15,7 @@ typedef unsigned short uint16_t;
 #endif
 
 #define DP_MAX_DIM 4
+#define DP_FF_PARAMS 5
 
 // Device status word shared by every kernel of one simulation handle. The host
 // reads it (pinned mirror) after each chunk of steps.
@@ -45,7 +46,8 @@ struct dp_pair_args {
     const double* sig_tab;
     const double* eps_tab;
     const double* isig_tab;  // 1 / sigma per type pair (DP_PMODE == 1)
-    const float2* ff_tab;    // DP_PMODE == 1: (sigma, 1/sigma, epsilon) as double-float triples
+    const float2* ff_tab;    // DP_PMODE == 1: per type pair DP_FF_PARAMS double-floats (see ff_const)
+    const float4* f32_tab;   // DP_PMODE == 1: per type pair sigma, 1/sigma, epsilon
     const void* pos64;       // 64-bit fixed-point positions (X = x 2^64 / L), one vector per particle
     const int32_t* order;    // particle id held by each slot (slots are in cell order after a rebuild)
     double* out;
@@ -64,8 +66,11 @@ struct dp_pair_args {
     double rcut;             // r_cut in units of sigma
     float cut2f;             // pre-filter: skip a pair when its float32 r^2 exceeds this
     float rcut_f;            // (float) rcut
+    float rcut2_f;           // (float) rcut^2
     int rcut_finite;
-    float ff_const[6];       // DP_PMODE == 0: sigma, 1/sigma, epsilon as double-float pairs
+    // DP_PMODE == 0: sigma, 1/sigma, epsilon, 1/sigma^2, epsilon/sigma as double-float pairs
+    float ff_const[2 * DP_FF_PARAMS];
+    float f32_const[4];      // DP_PMODE == 0: sigma, 1/sigma, epsilon
     int pad1;
 };
 

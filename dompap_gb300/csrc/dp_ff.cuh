@@ -100,20 +100,31 @@ __device__ __forceinline__ dpff dpff_add_f(dpff x, float b) {
     return dpff_quick_two_sum(s.hi, s.lo + x.lo);
 }
 
-// int64 -> double-float (rounded to ~48 bits) without 64-bit conversion
-// instructions: v = a 2^42 + b 2^20 + c with a in [-2^21, 2^21), b < 2^22,
-// c < 2^20, each piece an exact float. fa + fb is a multiple of 2^20 and
-// |fa| >= 2^42 > |fb| unless fa = 0, so Fast2Sum (QuickTwoSum) is exact for
-// it and again for adding fc (|fc| < 2^20 <= |fa + fb| unless that is 0).
-__device__ __forceinline__ dpff dpff_from_ll(long long v) {
-    const int a = (int)(v >> 42);
-    const int b = (int)(((unsigned long long)v >> 20) & 0x3FFFFFull);
-    const int c = (int)((unsigned long long)v & 0xFFFFFull);
-    const float fa = dp_small_int(a) * 4398046511104.0f;  // 2^42
-    const float fb = dp_small_int(b) * 1048576.0f;        // 2^20
-    const dpff ab = dpff_quick_two_sum(fa, fb);
-    const dpff t = dpff_quick_two_sum(ab.hi, dp_small_int(c));
-    return dpff_quick_two_sum(t.hi, t.lo + ab.lo);
+// 1/q: the float estimate y (one ulp, so e = 1 - q y below is ~2^-23; its
+// leading part 1 - q.hi y is exact by FMA), refined by y (1 + e + e^2):
+// ~2^-47 relative.
+__device__ __forceinline__ dpff dpff_rcp(dpff q) {
+    float y;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(q.hi));
+    const float e = fmaf(-q.lo, y, fmaf(-q.hi, y, 1.0f));
+    return dpff_quick_two_sum(y, y * fmaf(e, e, e));
+}
+
+// The 64-bit fixed-point displacement v (units 2^-64 L) times L, U = L / 2^32 as
+// a double-float, u24 = U.hi / 2^24. v = h 2^32 + l: the float of h rounded
+// towards zero leaves at most 7 bits of h, which with the upper 24 bits of l
+// make one 31-bit integer (a funnel shift), so three conversions carry ~48
+// leading bits of v; what is dropped lies below 2^-56 L. (An int64 split into
+// 22 / 22 / 20 bits took the same three conversions and twice the
+// instructions.)
+__device__ __forceinline__ dpff dpff_from_fixed(long long v, dpff U, float u24) {
+    const int h = (int)(v >> 32);
+    const float fh = __int2float_rz(h);
+    const int rest = h - __float2int_rz(fh);
+    const float fl = __int2float_rn((int)__funnelshift_l((uint32_t)v, (uint32_t)rest, 24));
+    const float p = fh * U.hi;
+    const float e = fmaf(fh, U.hi, -p);
+    return dpff_quick_two_sum(p, fmaf(fl, u24, fmaf(fh, U.lo, e)));
 }
 
 // Compensated accumulation s += v (cascaded summation in the manner of

@@ -44,14 +44,14 @@
 typedef DP_REAL real_t;
 typedef typename dp_shadow_t<DP_DIM>::type shadow_t;
 
-__device__ __forceinline__ void dp_pair_params(const dp_pair_args& a, long long i, int ti, int j, double& sig,
+// sigma, 1/sigma and epsilon of the pair of slots i and j, of types ti and tj.
+__device__ __forceinline__ void dp_pair_params(const dp_pair_args& a, long long i, int ti, int j, int tj, double& sig,
                                                double& isig, double& eps) {
 #if DP_PMODE == 0
     sig = a.sigma;
     isig = a.inv_sigma;
     eps = a.epsilon;
 #elif DP_PMODE == 1
-    const int tj = __ldg(a.types + j);
     sig = __ldg(a.sig_tab + ti * a.ntypes + tj);
     isig = __ldg(a.isig_tab + ti * a.ntypes + tj);
     eps = __ldg(a.eps_tab + ti * a.ntypes + tj);
@@ -89,6 +89,251 @@ __device__ __forceinline__ bool dp_upper_skip(const dp_pair_args& a, long long i
 #endif
 }
 
+// What a particle (or a lane of its group) has summed over its pairs.
+struct dp_pair_acc {
+    real_t v[DP_DIM];  // force: float32, or the float64 path of the parity mode
+    double s;          // energy, virial or Laplacian
+#if DP_FF
+    dpff fv[DP_DIM];   // compensated sums (dpff_accumulate)
+    dpff fs;
+    bool used64;
+#endif
+    __device__ __forceinline__ dp_pair_acc() : s(0.0) {
+#pragma unroll
+        for (int k = 0; k < DP_DIM; ++k) v[k] = real_t(0);
+#if DP_FF
+        used64 = false;
+#endif
+    }
+    // The scalar sum and, for DP_ACC_FORCE, the force vector.
+    template <int ACC>
+    __device__ __forceinline__ double finish(double* f) const {
+#if DP_FF
+        // double-float -> float64 by moving bits (one float64 add per value)
+        if (ACC == DP_ACC_FORCE) {
+#pragma unroll
+            for (int k = 0; k < DP_DIM; ++k)
+                f[k] = used64 ? (double)v[k] + dpff_to_double(fv[k]) : dpff_to_double(fv[k]);
+        }
+        return used64 ? s + dpff_to_double(fs) : dpff_to_double(fs);
+#else
+        if (ACC == DP_ACC_FORCE) {
+#pragma unroll
+            for (int k = 0; k < DP_DIM; ++k) f[k] = (double)v[k];
+        }
+        return s;
+#endif
+    }
+};
+
+// dp_pair_g (f(s)/s as a function of s^2: a double-float reciprocal and no
+// square root) where the potential has it; the force and the virial are the
+// sums that gain from it. With it and dpff_from_fixed a Lennard-Jones pair takes
+// about half the instructions: the mixture of 256,000 (skin 0.5) went from 434
+// to 388 us a step.
+#if defined(DP_PAIR_EVEN) && DP_FF
+#define DP_USES_G(ACC) ((ACC) == DP_ACC_FORCE || (ACC) == DP_ACC_VIRIAL)
+#else
+#define DP_USES_G(ACC) false
+#endif
+#ifndef DP_PAIR_EVEN
+template <typename R>
+__device__ __forceinline__ R dp_pair_g(R, R) {
+    return R(0);
+}
+#endif
+
+#if DP_REAL_IS_FLOAT
+// One pair in float32 on the fixed-point displacement df with q = |df|^2.
+// (dp_pair_g would save the square root's multiplication here but needs a
+// second comparison near the cut, where both forms have to decide alike: no
+// gain, 1.7 % slower on 500,000 LJ particles.)
+template <int ACC>
+__device__ __forceinline__ void dp_pair_eval(const dp_pair_args& a, long long i, int j, int ti, int tj, float q,
+                                             const float* df, dp_pair_acc& A) {
+    constexpr int D = DP_DIM;
+#if DP_PMODE == 0
+    const float sig = a.f32_const[0], isig = a.f32_const[1], e = a.f32_const[2];
+#elif DP_PMODE == 1
+    const float4 par = __ldg(a.f32_tab + ti * a.ntypes + tj);
+    const float sig = par.x, isig = par.y, e = par.z;
+#else
+    double sig64, isig64, eps64;
+    dp_pair_params(a, i, ti, j, tj, sig64, isig64, eps64);
+    const float sig = (float)sig64, isig = (float)isig64, e = (float)eps64;
+#endif
+    const float rinv = rsqrtf(q);
+    const float r = q * rinv;
+#if DP_SIGMA_ONE
+    const float s = r, sinv = rinv;
+#else
+    const float s = r * isig, sinv = rinv * sig;
+#endif
+    if (s > (float)a.rcut) return;
+    if (ACC == DP_ACC_FORCE) {
+#if DP_EPS_ONE
+        const float sf = dp_pair_f<float>(s, sinv);
+#else
+        const float sf = e * dp_pair_f<float>(s, sinv);
+#endif
+        const float g = sf * rinv;
+#pragma unroll
+        for (int k = 0; k < D; ++k) A.v[k] = fmaf(g, df[k], A.v[k]);
+    } else if (ACC == DP_ACC_ENERGY || ACC == DP_ACC_ENERGY_UPPER) {
+        A.s += (double)(e * dp_pair_u<float>(s, sinv));
+    } else if (ACC == DP_ACC_VIRIAL) {
+        A.s += (double)(e * dp_pair_f<float>(s, sinv) * r);
+    } else {
+        A.s += (double)(e * dp_pair_c<float>(s, sinv) + (float)(D - 1) * (-e * dp_pair_f<float>(s, sinv)) * rinv);
+    }
+}
+#endif
+
+#if DP_FF
+// One pair in double-float on the exact 64-bit fixed-point displacement.
+// False: the pair needs the float64 path (its scaled distance lies within float
+// rounding of r_cut, or is zero).
+template <int ACC>
+__device__ __forceinline__ bool dp_pair_eval_ff(const dp_pair_args& a, long long i, int j, int ti, int tj,
+                                                const unsigned long long* Xi, const unsigned long long* Xj,
+                                                dp_pair_acc& A) {
+    constexpr int D = DP_DIM;
+    dpff d[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        const dpff U(a.unit64_hi[k] * 4294967296.0f, a.unit64_lo[k] * 4294967296.0f);
+        d[k] = dpff_from_fixed((long long)(Xi[k] - Xj[k]), U, a.unit64_hi[k] * 256.0f);
+    }
+    dpff q = dpff_sqr_unnormalised(d[0]);
+#pragma unroll
+    for (int k = 1; k < D; ++k) dpff_accumulate(q, dpff_sqr_unnormalised(d[k]));
+    q = dpff_quick_two_sum(q.hi, q.lo);
+#if DP_PMODE == 0
+    const float* c = a.ff_const;
+    const dpff sig(c[0], c[1]), isig(c[2], c[3]), eps(c[4], c[5]), isig2(c[6], c[7]), eps_isig(c[8], c[9]);
+#elif DP_PMODE == 1
+    const float2* tri = a.ff_tab + DP_FF_PARAMS * (ti * a.ntypes + tj);
+    auto par = [&](int t) {
+        const float2 v = __ldg(tri + t);
+        return dpff(v.x, v.y);
+    };
+    const dpff sig = par(0), isig = par(1), eps = par(2);
+    const dpff isig2 = par(3), eps_isig = par(4);
+#else
+    double sig64, isig64, eps64;
+    dp_pair_params(a, i, ti, j, tj, sig64, isig64, eps64);
+    const dpff sig(sig64), isig(isig64), eps(eps64);
+    const dpff isig2 = isig * isig, eps_isig = eps * isig;
+#endif
+    if (DP_USES_G(ACC)) {
+#if DP_SIGMA_ONE
+        const dpff s2 = q;
+#else
+        const dpff s2 = q * isig2;
+#endif
+        if (a.rcut_finite && fabsf(s2.hi - a.rcut2_f) <= 2e-5f * a.rcut2_f) return false;
+        if (!(s2.hi > 0.0f)) return false;
+        if (s2.hi > a.rcut2_f) return true;
+        const dpff g = dp_pair_g<dpff>(s2, dpff_rcp(s2));
+        if (ACC == DP_ACC_FORCE) {
+#if DP_SIGMA_ONE && DP_EPS_ONE
+            const dpff h = g;
+#else
+            const dpff h = eps_isig * g;
+#endif
+#pragma unroll
+            for (int k = 0; k < D; ++k) dpff_accumulate_prod(A.fv[k], h, d[k]);
+        } else {
+            dpff_accumulate(A.fs, eps * sig * (g * s2));  // eps f(s) r, f = g s, r = sigma s
+        }
+        return true;
+    }
+    const dpff rinv = dpff_rsqrt(q);
+    const dpff r = q * rinv;
+#if DP_SIGMA_ONE
+    const dpff s = r, sinv = rinv;
+#else
+    const dpff s = r * isig, sinv = rinv * sig;
+#endif
+    if (a.rcut_finite && fabsf(s.hi - a.rcut_f) <= 1e-5f * a.rcut_f) return false;
+    if (s.hi > a.rcut_f) return true;
+    if (ACC == DP_ACC_FORCE) {
+#if DP_EPS_ONE
+        const dpff g = dp_pair_f<dpff>(s, sinv) * rinv;
+#else
+        const dpff g = eps * dp_pair_f<dpff>(s, sinv) * rinv;
+#endif
+#pragma unroll
+        for (int k = 0; k < D; ++k) dpff_accumulate_prod(A.fv[k], g, d[k]);
+    } else if (ACC == DP_ACC_ENERGY || ACC == DP_ACC_ENERGY_UPPER) {
+        dpff_accumulate(A.fs, eps * dp_pair_u<dpff>(s, sinv));
+    } else if (ACC == DP_ACC_VIRIAL) {
+        dpff_accumulate(A.fs, eps * dp_pair_f<dpff>(s, sinv) * r);
+    } else {
+        const dpff sf = eps * dp_pair_f<dpff>(s, sinv);
+        dpff_accumulate(A.fs, eps * dp_pair_c<dpff>(s, sinv) - dpff(D - 1) * sf * rinv);
+    }
+    return true;
+}
+#endif
+
+#if !DP_REAL_IS_FLOAT
+// One pair in float64 on the positions of slots i and j. d and r^2 follow the
+// reference exactly; 1/r comes from one reciprocal square root (no divisions),
+// and where s lies within a few ulp of r_cut, r = sqrt(r^2) and s = r / sigma
+// are recomputed with IEEE operations so the cut decision is the reference's.
+template <int ACC>
+__device__ __forceinline__ void dp_pair_eval_f64(const dp_pair_args& a, long long i, int j, int ti, int tj,
+                                                 dp_pair_acc& A) {
+    constexpr int D = DP_DIM;
+    const long long n = a.n;
+#if DP_FF
+    A.used64 = true;
+#endif
+    double sig, isig, eps;
+    dp_pair_params(a, i, ti, j, tj, sig, isig, eps);
+    double d[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) d[k] = dp_min_image(a.pos[k * n + i] - a.pos[k * n + j], a.box[k]);
+    const double q = dp_sqsum_exact<D>(d);
+    const double rinv = rsqrt(q);
+    double r = q * rinv;
+#if DP_SIGMA_ONE
+    double s = r;
+    const double sinv = rinv;
+#else
+    double s = r * isig;
+    const double sinv = rinv * sig;
+#endif
+    if (fabs(s - a.rcut) <= 1e-14 * a.rcut) {
+        r = sqrt(q);
+#if DP_SIGMA_ONE
+        s = r;
+#else
+        s = r / sig;
+#endif
+    }
+    if (s > a.rcut) return;
+    if (ACC == DP_ACC_FORCE) {
+#if DP_EPS_ONE
+        const double sf = dp_pair_f<double>(s, sinv);
+#else
+        const double sf = eps * dp_pair_f<double>(s, sinv);
+#endif
+        const double g = sf * rinv;
+#pragma unroll
+        for (int k = 0; k < D; ++k) A.v[k] = fma(g, d[k], A.v[k]);
+    } else if (ACC == DP_ACC_ENERGY || ACC == DP_ACC_ENERGY_UPPER) {
+        A.s += eps * dp_pair_u<double>(s, sinv);
+    } else if (ACC == DP_ACC_VIRIAL) {
+        A.s += eps * dp_pair_f<double>(s, sinv) * r;
+    } else {
+        const double sf = eps * dp_pair_f<double>(s, sinv);
+        A.s += eps * dp_pair_c<double>(s, sinv) + (double)(D - 1) * (-sf) * rinv;
+    }
+}
+#endif
+
 // Per-particle neighbour loop. Returns the scalar sum (energy / virial /
 // Laplacian) and, for DP_ACC_FORCE, the force vector in f[].
 //
@@ -113,23 +358,16 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
     const long long n = a.n;
     const shadow_t* __restrict__ sh = (const shadow_t*)a.shadow;
     uint32_t ui[D];
-    double xi[D];
     int ti = 0;
 #if DP_PMODE == 1
     ti = a.types[i];
 #endif
-    real_t acc_v[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) acc_v[k] = real_t(0);
-    double acc_s = 0.0;
+    dp_pair_acc A;
 #if DP_FF
     typedef typename dp_fixed64_t<D>::type fx_t;
     const fx_t* __restrict__ p64 = (const fx_t*)a.pos64;
     const bool ff_ok = a.status->far == 0;  // single-shift image == nearest image
     unsigned long long Xi[D];
-    dpff U[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) U[k] = dpff(a.unit64_hi[k], a.unit64_lo[k]);
     if (ff_ok) {
         // the pre-filter runs on the upper words of the 64-bit fixed point
         dp_fixed64_unpack<D>(p64[i], Xi);
@@ -137,24 +375,9 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
         for (int k = 0; k < D; ++k) ui[k] = (uint32_t)(Xi[k] >> 32);
     } else {
         dp_shadow_unpack<D>(sh[i], ui);
-#pragma unroll
-        for (int k = 0; k < D; ++k) xi[k] = a.pos[k * n + i];
     }
-    const float rcut_f = a.rcut_f;
-    const bool rcut_finite = a.rcut_finite != 0;
-    dpff facc[D];  // compensated sums (dpff_accumulate)
-    dpff sacc;
-    bool used64 = false;
-#if DP_PMODE == 0
-    const dpff sig_c(a.ff_const[0], a.ff_const[1]), isig_c(a.ff_const[2], a.ff_const[3]),
-        eps_c(a.ff_const[4], a.ff_const[5]);
-#endif
 #else
     dp_shadow_unpack<D>(sh[i], ui);
-#if !(DP_REAL_IS_FLOAT)
-#pragma unroll
-    for (int k = 0; k < D; ++k) xi[k] = a.pos[k * n + i];
-#endif
 #endif
     // Two passes over windows of up to 32 listed neighbours. Pass 1 runs the
     // float32 pre-filter on the shadows and keeps a bit per neighbour that
@@ -186,169 +409,29 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
             const int t = __ffs(kept) - 1;
             kept &= kept - 1;
             const int j = ALL ? (base + t) * LANES + lane : __ldg(row + (long long)(base + t) * entry_stride);
-            uint32_t uj[D];
-#if DP_FF
-            unsigned long long Xj[D];
-            if (ff_ok) {
-                dp_fixed64_unpack<D>(p64[j], Xj);
-#pragma unroll
-                for (int k = 0; k < D; ++k) uj[k] = (uint32_t)(Xj[k] >> 32);
-            } else {
-                dp_shadow_unpack<D>(__ldg(sh + j), uj);
-            }
-#else
-            dp_shadow_unpack<D>(__ldg(sh + j), uj);
+            int tj = 0;
+#if DP_PMODE == 1
+            tj = __ldg(a.types + j);
 #endif
+#if DP_REAL_IS_FLOAT
+            uint32_t uj[D];
+            dp_shadow_unpack<D>(__ldg(sh + j), uj);
             float df[D];
             const float qf = dp_shadow_q<D>(ui, uj, a.unit, df);
-#if DP_REAL_IS_FLOAT
-            double sig, isig, eps;
-            dp_pair_params(a, i, ti, j, sig, isig, eps);
-            // FP32 pair arithmetic on the fixed-point displacement.
-            const float rinv = rsqrtf(qf);
-            const float r = qf * rinv;
-#if DP_SIGMA_ONE
-            const float s = r, sinv = rinv;
-#else
-            const float s = r * (float)isig, sinv = rinv * (float)sig;
-#endif
-            if (s > (float)a.rcut) continue;
-            const float e = (float)eps;
-            if (ACC == DP_ACC_FORCE) {
-#if DP_EPS_ONE
-                const float sf = dp_pair_f<float>(s, sinv);
-#else
-                const float sf = e * dp_pair_f<float>(s, sinv);
-#endif
-                const float g = sf * rinv;
-#pragma unroll
-                for (int k = 0; k < D; ++k) acc_v[k] = fmaf(g, df[k], acc_v[k]);
-            } else if (ACC == DP_ACC_ENERGY || ACC == DP_ACC_ENERGY_UPPER) {
-                acc_s += (double)(e * dp_pair_u<float>(s, sinv));
-            } else if (ACC == DP_ACC_VIRIAL) {
-                acc_s += (double)(e * dp_pair_f<float>(s, sinv) * r);
-            } else {
-                acc_s += (double)(e * dp_pair_c<float>(s, sinv) + (float)(D - 1) * (-e * dp_pair_f<float>(s, sinv)) * rinv);
-            }
+            dp_pair_eval<ACC>(a, i, j, ti, tj, qf, df, A);
 #else
 #if DP_FF
             if (ff_ok) {
-                // double-float pair arithmetic on the exact fixed-point displacement
-                dpff d[D];
-#pragma unroll
-                for (int k = 0; k < D; ++k) d[k] = dpff_from_ll((long long)(Xi[k] - Xj[k])) * U[k];
-                dpff q = dpff_sqr_unnormalised(d[0]);
-#pragma unroll
-                for (int k = 1; k < D; ++k) dpff_accumulate(q, dpff_sqr_unnormalised(d[k]));
-                q = dpff_quick_two_sum(q.hi, q.lo);
-                const dpff rinv = dpff_rsqrt(q);
-                const dpff r = q * rinv;
-#if DP_PMODE == 0
-                const dpff fsig = sig_c, fisig = isig_c, feps = eps_c;
-#elif DP_PMODE == 1
-                const int tj = __ldg(a.types + j);
-                const float2* tri = a.ff_tab + 3 * (ti * a.ntypes + tj);
-                const float2 t0 = __ldg(tri), t1 = __ldg(tri + 1), t2 = __ldg(tri + 2);
-                const dpff fsig(t0.x, t0.y), fisig(t1.x, t1.y), feps(t2.x, t2.y);
-#else
-                double sig, isig, eps;
-                dp_pair_params(a, i, ti, j, sig, isig, eps);
-                const dpff fsig(sig), fisig(isig), feps(eps);
-#endif
-#if DP_SIGMA_ONE
-                const dpff s = r, sinv = rinv;
-#else
-                const dpff s = r * fisig, sinv = rinv * fsig;
-#endif
-                if (!(rcut_finite && fabsf(s.hi - rcut_f) <= 1e-5f * rcut_f)) {
-                    if (s.hi > rcut_f) continue;
-                    if (ACC == DP_ACC_FORCE) {
-#if DP_EPS_ONE
-                        const dpff g = dp_pair_f<dpff>(s, sinv) * rinv;
-#else
-                        const dpff g = feps * dp_pair_f<dpff>(s, sinv) * rinv;
-#endif
-#pragma unroll
-                        for (int k = 0; k < D; ++k) dpff_accumulate_prod(facc[k], g, d[k]);
-                    } else if (ACC == DP_ACC_ENERGY || ACC == DP_ACC_ENERGY_UPPER) {
-                        dpff_accumulate(sacc, feps * dp_pair_u<dpff>(s, sinv));
-                    } else if (ACC == DP_ACC_VIRIAL) {
-                        dpff_accumulate(sacc, feps * dp_pair_f<dpff>(s, sinv) * r);
-                    } else {
-                        const dpff sf = feps * dp_pair_f<dpff>(s, sinv);
-                        dpff_accumulate(sacc, feps * dp_pair_c<dpff>(s, sinv) - dpff(D - 1) * sf * rinv);
-                    }
-                    continue;
-                }
-                // within float rounding of r_cut: the float64 path below
-#pragma unroll
-                for (int k = 0; k < D; ++k) xi[k] = a.pos[k * n + i];
+                unsigned long long Xj[D];
+                dp_fixed64_unpack<D>(p64[j], Xj);
+                if (dp_pair_eval_ff<ACC>(a, i, j, ti, tj, Xi, Xj, A)) continue;
             }
-            used64 = true;
 #endif
-            // FP64 pair arithmetic. d and r^2 follow the reference exactly; 1/r
-            // comes from one reciprocal square root (no divisions), and where s
-            // lies within a few ulp of r_cut, r = sqrt(r^2) and s = r / sigma are
-            // recomputed with IEEE operations so the cut decision is the
-            // reference's.
-            double sig, isig, eps;
-            dp_pair_params(a, i, ti, j, sig, isig, eps);
-            double d[D];
-#pragma unroll
-            for (int k = 0; k < D; ++k) d[k] = dp_min_image(xi[k] - __ldg(a.pos + k * n + j), a.box[k]);
-            const double q = dp_sqsum_exact<D>(d);
-            const double rinv = rsqrt(q);
-            double r = q * rinv;
-#if DP_SIGMA_ONE
-            double s = r;
-            const double sinv = rinv;
-#else
-            double s = r * isig;
-            const double sinv = rinv * sig;
-#endif
-            if (fabs(s - a.rcut) <= 1e-14 * a.rcut) {
-                r = sqrt(q);
-#if DP_SIGMA_ONE
-                s = r;
-#else
-                s = r / sig;
-#endif
-            }
-            if (s > a.rcut) continue;
-            if (ACC == DP_ACC_FORCE) {
-#if DP_EPS_ONE
-                const double sf = dp_pair_f<double>(s, sinv);
-#else
-                const double sf = eps * dp_pair_f<double>(s, sinv);
-#endif
-                const double g = sf * rinv;
-#pragma unroll
-                for (int k = 0; k < D; ++k) acc_v[k] = fma(g, d[k], acc_v[k]);
-            } else if (ACC == DP_ACC_ENERGY || ACC == DP_ACC_ENERGY_UPPER) {
-                acc_s += eps * dp_pair_u<double>(s, sinv);
-            } else if (ACC == DP_ACC_VIRIAL) {
-                acc_s += eps * dp_pair_f<double>(s, sinv) * r;
-            } else {
-                const double sf = eps * dp_pair_f<double>(s, sinv);
-                acc_s += eps * dp_pair_c<double>(s, sinv) + (double)(D - 1) * (-sf) * rinv;
-            }
+            dp_pair_eval_f64<ACC>(a, i, j, ti, tj, A);
 #endif
         }
     }
-#if DP_FF
-    // double-float -> float64 by moving bits (one float64 add per value)
-    if (ACC == DP_ACC_FORCE) {
-#pragma unroll
-        for (int k = 0; k < D; ++k) f[k] = used64 ? (double)acc_v[k] + dpff_to_double(facc[k]) : dpff_to_double(facc[k]);
-    }
-    return used64 ? acc_s + dpff_to_double(sacc) : dpff_to_double(sacc);
-#else
-    if (ACC == DP_ACC_FORCE) {
-#pragma unroll
-        for (int k = 0; k < D; ++k) f[k] = (double)acc_v[k];
-    }
-    return acc_s;
-#endif
+    return A.template finish<ACC>(f);
 }
 
 // F (SoA float64) for every particle. One thread per particle; the
