@@ -8,7 +8,7 @@ derived symbolically, and the three are printed as templated device functions
     template <typename R> __device__ R dp_pair_f(R r, R dp_inv_r);   // -du/dr
     template <typename R> __device__ R dp_pair_c(R r, R dp_inv_r);   // d2u/dr2
 
-and, where ``u`` has only even powers of ``r`` (Lennard-Jones and its kin),
+and, where ``-u'/r`` is a polynomial in ``r**2`` and ``r**-2`` (Lennard-Jones and its kin),
 
     #define DP_PAIR_EVEN 1
     template <typename R> __device__ R dp_pair_g(R q, R dp_inv_q);   // -du/dr / r at q = r^2

@@ -1,4 +1,5 @@
-"""dp_pair_g, the generated f(r)/r of potentials with only even powers of r:
+"""dp_pair_g, the generated f(r)/r of potentials whose f/r is a polynomial in
+r^2 and 1/r^2 (even powers of r; also a logarithm, whose force is -1/r):
 present exactly for those, and equal to dp_pair_f(r)/r (both compiled for the
 host in double) over the distances a pair loop meets."""
 import re
@@ -10,9 +11,10 @@ import pytest
 from dompap_gb300 import codegen
 
 EVEN = ["4*(r**-12-r**-6)", "r**2/2 + 0.1*r**-4", "1-r**2", "2.5*r**4 - 3/r**2", "0*r", "3*(r**-10 - 0.7*r**-2)",
-        "r**-64 + 1e-3*r**64"]
+        "r**-64 + 1e-3*r**64",
+        "log(r)"]
 ODD = ["(1-r)**2", "r**-9 - r**-6", "4*(r**-12-r**-6) + exp(-r)", "r**-12 - (r - 2.5)", "sqrt(r)", "cos(r**2)",
-       "r**-130", "1/(1+r**2)", "log(r)"]
+       "r**-130", "1/(1+r**2)", "r*log(r)"]
 
 HARNESS = r"""
 #include <cmath>
