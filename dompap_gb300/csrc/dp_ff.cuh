@@ -92,7 +92,7 @@ __device__ __forceinline__ dpff dpff_rsqrt(dpff q) {
 // x^2 unnormalised: (p, e) with p + e = x^2 to ~2^-48 (for dpff_accumulate).
 __device__ __forceinline__ dpff dpff_sqr_unnormalised(dpff x) {
     const float p = x.hi * x.hi;
-    return dpff(p, fmaf(x.hi + x.hi, x.lo, fmaf(x.hi, x.hi, -p)));
+    return dpff(p, fmaf(fmaf(2.0f, x.hi, x.lo), x.lo, fmaf(x.hi, x.hi, -p)));
 }
 
 __device__ __forceinline__ dpff dpff_add_f(dpff x, float b) {
@@ -111,17 +111,20 @@ __device__ __forceinline__ dpff dpff_rcp(dpff q) {
 }
 
 // The 64-bit fixed-point displacement v (units 2^-64 L) times L, U = L / 2^32 as
-// a double-float, u24 = U.hi / 2^24. v = h 2^32 + l: the float of h rounded
-// towards zero leaves at most 7 bits of h, which with the upper 24 bits of l
-// make one 31-bit integer (a funnel shift), so three conversions carry ~48
-// leading bits of v; what is dropped lies below 2^-56 L. (An int64 split into
-// 22 / 22 / 20 bits took the same three conversions and twice the
-// instructions.)
+// a double-float, u24 = U.hi / 2^24. v = h 2^32 + l: what the nearest float of h
+// leaves of it (at most 64) and the upper 24 bits of l make one 31-bit integer
+// (a funnel shift), so three conversions carry ~48 leading bits of v; what is
+// dropped lies below 2^-56 L. An h that rounds up to 2^31 saturates on the way
+// back, one short of it. (An int64 split into 22 / 22 / 20 bits took the same
+// three conversions and twice the instructions; rounding h towards zero, or
+// leaving the product unnormalised, saves a few but costs a bit of accuracy.)
 __device__ __forceinline__ dpff dpff_from_fixed(long long v, dpff U, float u24) {
     const int h = (int)(v >> 32);
-    const float fh = __int2float_rz(h);
-    const int rest = h - __float2int_rz(fh);
-    const float fl = __int2float_rn((int)__funnelshift_l((uint32_t)v, (uint32_t)rest, 24));
+    const float fh = __int2float_rn(h);
+    int back = __float2int_rn(fh);
+    if (back == 0x7FFFFFFF) back = (int)0x80000000u;
+    const uint32_t rest = (uint32_t)h - (uint32_t)back;
+    const float fl = __int2float_rn((int)__funnelshift_l((uint32_t)v, rest, 24));
     const float p = fh * U.hi;
     const float e = fmaf(fh, U.hi, -p);
     return dpff_quick_two_sum(p, fmaf(fl, u24, fmaf(fh, U.lo, e)));
