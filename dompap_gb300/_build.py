@@ -43,7 +43,7 @@ def write_embedded() -> str:
     for name, sym in (("dp_common.cuh", "dp_src_common"), ("pair_kernels.cuh", "dp_src_pair"),
                       ("batch_kernels.cuh", "dp_src_batch"), ("mlp_common.cuh", "dp_src_mlp"),
                       ("dp_ff.cuh", "dp_src_ff"), ("dp_integrate.cuh", "dp_src_integrate"),
-                      ("dp_umma.cuh", "dp_src_umma")):
+                      ("dp_umma.cuh", "dp_src_umma"), ("brick_kernels.cuh", "dp_src_brick")):
         with open(os.path.join(CSRC, name)) as fh:
             text = fh.read()
         if ')DPSRC"' in text:
@@ -99,6 +99,8 @@ def check_pair_kernels(verbose: bool = True) -> None:
         common = fh.read()
     with open(os.path.join(CSRC, "pair_kernels.cuh")) as fh:
         pair = fh.read()
+    with open(os.path.join(CSRC, "brick_kernels.cuh")) as fh:
+        brick = fh.read()
     with open(os.path.join(CSRC, "batch_kernels.cuh")) as fh:
         batch = fh.read()
     with open(os.path.join(CSRC, "dp_ff.cuh")) as fh:
@@ -111,7 +113,7 @@ def check_pair_kernels(verbose: bool = True) -> None:
                 src = (f"#define DP_DIM {dim}\n#define DP_REAL {real}\n#define DP_REAL_IS_FLOAT {is_float}\n"
                        f"#define DP_PMODE {pmode}\n#define DP_SIGMA_ONE {int(pmode == 0)}\n"
                        f"#define DP_EPS_ONE {int(pmode == 0)}\n#define DP_FF {1 - is_float}\n#include <cstdint>\n"
-                       + common + integ + (ffsrc if not is_float else "") + SAMPLE_POTENTIAL + pair
+                       + common + integ + (ffsrc if not is_float else "") + SAMPLE_POTENTIAL + pair + brick
                        + (batch if is_float and pmode == 0 else ""))
                 path = os.path.join(BUILD, f"pair_check_{dim}_{real}_{pmode}.cu")
                 with open(path, "w") as fh:

@@ -22,7 +22,7 @@ typedef unsigned short uint16_t;
 struct dp_dev_status {
     int32_t need_rebuild;     // 1: the next step rebuilds the neighbour list
     int32_t max_neighbors;    // largest neighbour count seen by the last build
-    int32_t cell_overflow;    // largest cell occupancy seen when it exceeded capacity
+    int32_t cell_overflow;    // largest brick region seen when it exceeded its capacity
     int32_t nonfinite;        // a force or position became NaN/Inf
     int32_t far;              // some coordinate lies outside [-L/4, 5L/4) (not yet wrapped)
     int32_t device_error;     // a bounded device-side wait gave up: the launch's results are invalid
@@ -71,6 +71,13 @@ struct dp_pair_args {
     // DP_PMODE == 0: sigma, 1/sigma, epsilon, 1/sigma^2, epsilon/sigma as double-float pairs
     float ff_const[2 * DP_FF_PARAMS];
     float f32_const[4];      // DP_PMODE == 0: sigma, 1/sigma, epsilon
+    // bricks (brick_kernels.cuh): per brick (first slot, particles, region
+    // entries, 0), the slots of its region (brick_cap per brick) and the lists
+    // (8 region indices per 16-byte chunk, chunk c of slot i at [c n + i])
+    const int4* brick_info;
+    const int32_t* brick_slots;
+    const uint4* brick_list;
+    int brick_cap;
     int pad1;
 };
 

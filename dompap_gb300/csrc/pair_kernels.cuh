@@ -127,12 +127,12 @@ struct dp_pair_acc {
 };
 
 // dp_pair_g (f(s)/s as a function of s^2: a double-float reciprocal and no
-// square root) where the potential has it; the force and the virial are the
-// sums that gain from it. With it and dpff_from_fixed a Lennard-Jones pair takes
+// square root) where the potential has it, for the forces (the virial would
+// lose a bit: its sum cancels). With it and dpff_from_fixed a Lennard-Jones pair takes
 // about half the instructions: the mixture of 256,000 (skin 0.5) went from 434
 // to 388 us a step.
 #if defined(DP_PAIR_EVEN) && DP_FF
-#define DP_USES_G(ACC) ((ACC) == DP_ACC_FORCE || (ACC) == DP_ACC_VIRIAL)
+#define DP_USES_G(ACC) ((ACC) == DP_ACC_FORCE)
 #else
 #define DP_USES_G(ACC) false
 #endif
@@ -144,6 +144,14 @@ __device__ __forceinline__ R dp_pair_g(R, R) {
 #endif
 
 #if DP_REAL_IS_FLOAT
+// 1/sqrt of a squared distance, without rsqrtf's scaling of subnormals: a pair
+// as close as 1e-19 overflows its force anyway.
+__device__ __forceinline__ float dp_rsqrt_normal(float q) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(q));
+    return y;
+}
+
 // One pair in float32 on the fixed-point displacement df with q = |df|^2.
 // (dp_pair_g would save the square root's multiplication here but needs a
 // second comparison near the cut, where both forms have to decide alike: no
@@ -162,14 +170,14 @@ __device__ __forceinline__ void dp_pair_eval(const dp_pair_args& a, long long i,
     dp_pair_params(a, i, ti, j, tj, sig64, isig64, eps64);
     const float sig = (float)sig64, isig = (float)isig64, e = (float)eps64;
 #endif
-    const float rinv = rsqrtf(q);
+    const float rinv = dp_rsqrt_normal(q);
     const float r = q * rinv;
 #if DP_SIGMA_ONE
     const float s = r, sinv = rinv;
 #else
     const float s = r * isig, sinv = rinv * sig;
 #endif
-    if (s > (float)a.rcut) return;
+    if (s > a.rcut_f) return;
     if (ACC == DP_ACC_FORCE) {
 #if DP_EPS_ONE
         const float sf = dp_pair_f<float>(s, sinv);
@@ -235,17 +243,13 @@ __device__ __forceinline__ bool dp_pair_eval_ff(const dp_pair_args& a, long long
         if (!(s2.hi > 0.0f)) return false;
         if (s2.hi > a.rcut2_f) return true;
         const dpff g = dp_pair_g<dpff>(s2, dpff_rcp(s2));
-        if (ACC == DP_ACC_FORCE) {
 #if DP_SIGMA_ONE && DP_EPS_ONE
-            const dpff h = g;
+        const dpff h = g;
 #else
-            const dpff h = eps_isig * g;
+        const dpff h = eps_isig * g;
 #endif
 #pragma unroll
-            for (int k = 0; k < D; ++k) dpff_accumulate_prod(A.fv[k], h, d[k]);
-        } else {
-            dpff_accumulate(A.fs, eps * sig * (g * s2));  // eps f(s) r, f = g s, r = sigma s
-        }
+        for (int k = 0; k < D; ++k) dpff_accumulate_prod(A.fv[k], h, d[k]);
         return true;
     }
     const dpff rinv = dpff_rsqrt(q);
@@ -334,6 +338,12 @@ __device__ __forceinline__ void dp_pair_eval_f64(const dp_pair_args& a, long lon
 }
 #endif
 
+// Window of the two-pass loop: one thread per particle evaluates 64 listed
+// neighbours at a time (mixture of 256,000, 150 listed: 320 / 298 / 307 us a
+// step with 32 / 64 / 128; 108,000 LJ, 95 listed: 91 / 87 / 84; lists of a
+// dozen: equal; 10 us more each with the displacement in its present form).
+#define DP_WINDOW 64
+
 // Per-particle neighbour loop. Returns the scalar sum (energy / virial /
 // Laplacian) and, for DP_ACC_FORCE, the force vector in f[].
 //
@@ -379,36 +389,55 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
 #else
     dp_shadow_unpack<D>(sh[i], ui);
 #endif
-    // Two passes over windows of up to 32 listed neighbours. Pass 1 runs the
-    // float32 pre-filter on the shadows and keeps a bit per neighbour that
+    // Two passes over windows of up to DP_WINDOW listed neighbours. Pass 1 runs
+    // the float32 pre-filter on the shadows and keeps a bit per neighbour that
     // may lie within r_cut * sigma_max; pass 2 evaluates the pair terms of
     // the kept ones only, in list order. A warp then runs the pair arithmetic
     // as often as its busiest lane has kept neighbours, not once per listed
-    // one (in a dense liquid with a thin skin most listed neighbours of most
-    // lanes are outside r_cut at any step).
+    // one, and the wider the window the closer the busiest lane is to the
+    // average (in a liquid about 73 % of the lanes are busy with 32, 79 % with 64).
     const int c_all = ALL ? (int)n : a.cnt[i];
     const int c = LANES > 1 ? (c_all > lane ? (c_all - lane + LANES - 1) / LANES : 0) : c_all;
     const int32_t* __restrict__ row = ALL ? nullptr : a.nl + i + (LANES > 1 ? (long long)lane * n : 0LL);
     const long long entry_stride = (long long)LANES * n;
-    for (int base = 0; base < c; base += 32) {
-        const int w = min(32, c - base);
-        uint32_t kept = 0;
+    constexpr int W = LANES > 1 ? 1 : DP_WINDOW / 32;  // words of a window
+    for (int base = 0; base < c; base += 32 * W) {
+        uint32_t kept[W];
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+            const int first = base + 32 * q, w = min(32, c - first);
+            kept[q] = 0u;
 #pragma unroll 4
-        for (int t = 0; t < w; ++t) {
-            const int j = ALL ? (base + t) * LANES + lane : __ldg(row + (long long)(base + t) * entry_stride);
-            if (ALL && j == i) continue;
-            // the virial and the double-loop energy are upper-triangle sums
-            // over n < m with sigma(n, m), epsilon(n, m)
-            if ((ACC == DP_ACC_VIRIAL || ACC == DP_ACC_ENERGY_UPPER) && dp_upper_skip(a, i, j)) continue;
-            uint32_t uj[D];
-            dp_shadow_unpack<D>(__ldg(sh + j), uj);
-            float df[D];
-            if (dp_shadow_q<D>(ui, uj, a.unit, df) <= a.cut2f) kept |= 1u << t;
+            for (int t = 0; t < w; ++t) {
+                const int j = ALL ? (first + t) * LANES + lane : __ldg(row + (long long)(first + t) * entry_stride);
+                if (ALL && j == i) continue;
+                // the virial and the double-loop energy are upper-triangle sums
+                // over n < m with sigma(n, m), epsilon(n, m)
+                if ((ACC == DP_ACC_VIRIAL || ACC == DP_ACC_ENERGY_UPPER) && dp_upper_skip(a, i, j)) continue;
+                uint32_t uj[D];
+                dp_shadow_unpack<D>(__ldg(sh + j), uj);
+                float df[D];
+                if (dp_shadow_q<D>(ui, uj, a.unit, df) <= a.cut2f) kept[q] |= 1u << t;
+            }
         }
-        while (kept) {
-            const int t = __ffs(kept) - 1;
-            kept &= kept - 1;
-            const int j = ALL ? (base + t) * LANES + lane : __ldg(row + (long long)(base + t) * entry_stride);
+        int first = base;
+        while (true) {
+            if (W > 1) {
+                // the next word with a bit; each lane on its own
+#pragma unroll
+                for (int q = 1; q < W; ++q) {
+                    if (kept[0] == 0u) {
+                        first += 32;
+#pragma unroll
+                        for (int p = 0; p + 1 < W; ++p) kept[p] = kept[p + 1];
+                        kept[W - 1] = 0u;
+                    }
+                }
+            }
+            if (kept[0] == 0u) break;
+            const int t = __ffs(kept[0]) - 1;
+            kept[0] &= kept[0] - 1;
+            const int j = ALL ? (first + t) * LANES + lane : __ldg(row + (long long)(first + t) * entry_stride);
             int tj = 0;
 #if DP_PMODE == 1
             tj = __ldg(a.types + j);
