@@ -527,6 +527,7 @@ struct NlArgs {
     const int32_t* src_of;     // slot of each entry of the ranges (null: the entries are the slots)
     dp_dev_status* st;
     long long n;
+    long long nl_k, nl_i;      // entry k of slot i at nl[k nl_k + i nl_i]
     int kcap;
     int morton;
     int nc[DP_MAX_DIM];
@@ -605,7 +606,7 @@ __global__ void __launch_bounds__(kBlock) k_nl_build_cells(NlArgs a) {
                 inside = sqrt(dp_sqsum_exact<D>(d)) < a.cutoff;
             }
             if (inside) {
-                if (count < a.kcap) a.nl[(long long)count * n + i] = j;
+                if (count < a.kcap) a.nl[count * a.nl_k + i * a.nl_i] = j;
                 ++count;
             }
         }
@@ -922,8 +923,8 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_brick_build(NlArgs a, Bric
                 found[h] += __shfl_sync(0xffffffffu, upto, 3, 4);
                 int left = min(mine, a.kcap - at);
                 if (OUT32) {
-                    int32_t* to = a.nl + (long long)at * n + i;
-                    for (; left > 0; --left, to += n) {
+                    int32_t* to = a.nl + at * a.nl_k + i * a.nl_i;
+                    for (; left > 0; --left, to += a.nl_k) {
                         const int s = __clz(m);
                         m &= ~(0x80000000u >> s);
                         *to = rslot[t0 + 8 * (s >> 1) + 2 * c + (s & 1)];
@@ -1019,7 +1020,7 @@ __global__ void __launch_bounds__(kBlock) k_nl_build_allpairs(NlArgs a) {
                     inside = sqrt(dp_sqsum_exact<D>(d)) < a.cutoff;
                 }
                 if (inside) {
-                    if (count < a.kcap) a.nl[(long long)count * n + i] = (int32_t)j;
+                    if (count < a.kcap) a.nl[count * a.nl_k + i * a.nl_i] = (int32_t)j;
                     ++count;
                 }
             }
@@ -1032,6 +1033,55 @@ __global__ void __launch_bounds__(kBlock) k_nl_build_allpairs(NlArgs a) {
 #pragma unroll
     for (int k = 0; k < D; ++k) a.pos_ref[k * n + i] = xi[k];
     ((sh_t*)a.shadow_ref)[i] = sh[i];
+}
+
+// Lists of small systems (a warp per particle; full or half, in rows or
+// columns): every other particle tested, 32 at a time, with the same decisions,
+// in ascending order. No cells, and the slots keep their order. A rebuild of 500
+// LJ particles 82 -> 15 us, of 4,000 434 -> 43 (one thread per particle before).
+template <int D>
+__global__ void __launch_bounds__(kBlock) k_nl_build_rows(NlArgs a) {
+    if (!a.st->need_rebuild) return;
+    typedef typename dp_shadow_t<D>::type sh_t;
+    const long long n = a.n;
+    const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= n) return;  // uniform across the warp
+    const bool far = a.st->far != 0;
+    const sh_t* __restrict__ sh = (const sh_t*)a.shadow;
+    const sh_t shi = sh[i];
+    uint32_t ui[D];
+    dp_shadow_unpack<D>(shi, ui);
+    int32_t* row = a.nl + i * a.nl_i;
+    int found = 0;
+#pragma unroll 2
+    for (int base = 0; base < (int)n; base += 32) {
+        const int j = base + lane;
+        bool in = false;
+        if (j < (int)n && (a.half ? dp_owns_pair(i, j) : j != (int)i)) {
+            uint32_t uj[D];
+            dp_shadow_unpack<D>(__ldg(sh + j), uj);
+            float df[D];
+            const float q = dp_shadow_q<D>(ui, uj, a.unit, df);
+            in = q <= a.hi2;
+            if (in && (far || !(q < a.lo2))) {
+                double d[D];
+#pragma unroll
+                for (int k = 0; k < D; ++k) d[k] = dp_min_image(a.pos[k * n + i] - a.pos[k * n + j], a.box[k]);
+                in = sqrt(dp_sqsum_exact<D>(d)) < a.cutoff;
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        const int at = found + __popc(m & ((1u << lane) - 1u));
+        if (in && at < a.kcap) row[at * a.nl_k] = j;
+        found += __popc(m);
+    }
+    if (lane == 0) {
+        a.cnt[i] = min(found, a.kcap);
+        ((sh_t*)a.shadow_ref)[i] = shi;
+        atomicMax(&a.st->max_neighbors, found);
+    }
+    if (lane < D) a.pos_ref[lane * n + i] = a.pos[lane * n + i];
 }
 
 // Self-test of the bounded device-side waits, without a GPU fault: one CTA
@@ -1079,12 +1129,12 @@ __global__ void k_advance_step(dp_dev_status* st, long long steps, int clear_far
     if (clear_far) st->far = 0;
 }
 
-// Rows of the column-major list (in slots) -> row-major (N, kout) by particle
+// The list of slots (entry k of slot r at k nl_k + r nl_i) -> row-major (N, kout) by particle
 // id, entries as particle ids, each row sorted ascending and -1 padded
 // (dompap's neighbor_list layout).
 __global__ void k_nl_export(const int32_t* __restrict__ nl, const int32_t* __restrict__ cnt, int32_t* out,
                             const int32_t* __restrict__ order, const int32_t* __restrict__ slot_of, long long n,
-                            int kout) {
+                            long long nl_k, long long nl_i, int kout) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const long long r = slot_of[i];
@@ -1092,7 +1142,7 @@ __global__ void k_nl_export(const int32_t* __restrict__ nl, const int32_t* __res
     int32_t* row = out + i * kout;
     int m = 0;  // entries kept so far (<= kout), the kout smallest in ascending order
     for (int k = 0; k < c; ++k) {
-        const int32_t v = order[nl[(long long)k * n + r]];
+        const int32_t v = order[nl[k * nl_k + r * nl_i]];
         int u;
         if (m < kout) {
             u = m - 1;
@@ -1157,7 +1207,7 @@ __global__ void __launch_bounds__(kBlock) k_integrate(dp_int_args a) {
         double F[D];
 #pragma unroll
         for (int k = 0; k < D; ++k) F[k] = a.force[k * a.n + i];
-        old = dp_integrate_one<D, MASSMODE, NVE, WRITE64>(a, i, F, bad);
+        old = dp_integrate_one<D, MASSMODE, NVE, WRITE64>(a, i, F, bad, -1);
     }
     const bool any_old = __any_sync(0xffffffffu, old);
     const bool any_bad = __any_sync(0xffffffffu, bad);
@@ -1478,6 +1528,9 @@ struct PairLib {
     cudaKernel_t step = nullptr;  // fused forces + integrate (not in the surrogate program)
     cudaKernel_t step_warp = nullptr;  // the same, one warp per particle (small systems)
     cudaKernel_t step_quad = nullptr;  // the same, four lanes per particle
+    cudaKernel_t step_lists = nullptr;  // one warp per particle, which rebuilds its own list
+    // sums with 32 (0) or 4 (1) lanes per particle: forces, energy, virial, Laplacian
+    cudaKernel_t split[2][4] = {{nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}};
     // no neighbour list (dompap's double-loop methods): fused step, forces, energy
     cudaKernel_t step_all = nullptr, forces_all = nullptr, energy_all = nullptr;
     // bricks of cells (not in 4-D, with dense parameters or in the surrogate
@@ -1643,6 +1696,12 @@ static int compile_pair_lib(const std::string& src, PairLib* out) {
         CK(cudaLibraryGetKernel(&pl.step, pl.lib, "dp_step"));
         CK(cudaLibraryGetKernel(&pl.step_warp, pl.lib, "dp_step_warp"));
         CK(cudaLibraryGetKernel(&pl.step_quad, pl.lib, "dp_step_quad"));
+        CK(cudaLibraryGetKernel(&pl.step_lists, pl.lib, "dp_step_lists"));
+        const char* quantity[4] = {"dp_forces_", "dp_energy_", "dp_virial_", "dp_laplacian_"};
+        for (int q = 0; q < 4; ++q) {
+            CK(cudaLibraryGetKernel(&pl.split[0][q], pl.lib, (std::string(quantity[q]) + "warp").c_str()));
+            CK(cudaLibraryGetKernel(&pl.split[1][q], pl.lib, (std::string(quantity[q]) + "quad").c_str()));
+        }
         CK(cudaLibraryGetKernel(&pl.step_all, pl.lib, "dp_step_all"));
         CK(cudaLibraryGetKernel(&pl.forces_all, pl.lib, "dp_forces_all"));
         CK(cudaLibraryGetKernel(&pl.energy_all, pl.lib, "dp_energy_all"));
@@ -1768,6 +1827,7 @@ struct dp_sim {
     double r_cut = 1.0;
     PairLib lib;
     bool lib_valid = false;
+    bool lib_sets_cond = false;  // the program sets graph conditions (want_cond)
 
     // pair surrogate (DP_PREC_MLP)
     const dp_mlp_dev* mlp_dev = nullptr;
@@ -2165,14 +2225,14 @@ static void fill_perm_args(const dp_sim* s, PermArgs& p) {
 }
 
 // The gated rebuild sequence (no effect unless need_rebuild is set).
-// What the lists hold: slots, every partner or only the owned ones
-// (dp_owns_pair; the surrogate mode uses each pair once), or region indices for
-// the brick kernels.
-enum { kListFull = 0, kListHalf = 1, kListBrick = 2 };
+// What the lists hold: slots, column-major, every partner or only the owned ones
+// (dp_owns_pair; the surrogate mode uses each pair once); slots in rows, where a
+// warp shares a particle; or region indices for the brick kernels.
+enum { kListFull = 0, kListHalf = 1, kListBrick = 2, kListRows = 3 };
 static int list_kind(const dp_sim* s) {
     if (s->precision == DP_PREC_MLP) return kListHalf;
     if (s->brick_pairs && s->step_lanes != 32 && s->lib.forces_brick) return kListBrick;
-    return kListFull;
+    return s->n <= s->warp_step_max ? kListRows : kListFull;
 }
 
 template <int D>
@@ -2219,13 +2279,23 @@ static int launch_rebuild(dp_sim* s, long long* launches) {
     na.cnt = s->cnt;
     na.st = s->dstat;
     na.n = s->n;
+    na.nl_k = list_kind(s) == kListRows ? 1 : s->n;
+    na.nl_i = list_kind(s) == kListRows ? s->kcap : 1;
     na.kcap = s->kcap;
     na.cutoff = s->cutoff;
     bracket(s, s->cutoff, &na.lo2, &na.hi2);
     fill_scale(s, nullptr, na.unit);
     for (int k = 0; k < DP_MAX_DIM; ++k) na.box[k] = (k < s->dim) ? s->box[k] : 1.0;
     long long nl_launches = 0;
-    if (s->use_cells) {
+    if (s->n <= s->warp_step_max) {
+        const unsigned gr = grid_for(s->n * 32, kBlock);
+        switch (s->dim) {
+            case 2: k_nl_build_rows<2><<<gr, kBlock, 0, s->stream>>>(na); break;
+            case 3: k_nl_build_rows<3><<<gr, kBlock, 0, s->stream>>>(na); break;
+            default: k_nl_build_rows<4><<<gr, kBlock, 0, s->stream>>>(na); break;
+        }
+        nl_launches = 1;
+    } else if (s->use_cells) {
         // counting sort of the slots by cell key
         BinArgs ba{};
         ba.shadow = s->shadow;
@@ -2322,6 +2392,8 @@ static void fill_pair_args(const dp_sim* s, dp_pair_args& a, double* out) {
     a.f32_tab = s->f32_tab;
     a.pos64 = s->pos64;
     a.order = s->order;
+    a.nl_k = list_kind(s) == kListRows ? 1 : s->n;
+    a.nl_i = list_kind(s) == kListRows ? s->kcap : 1;
     a.brick_info = s->brick_info;
     a.brick_slots = s->brick_slots;
     a.brick_list = (const uint4*)s->nl;
@@ -2377,6 +2449,14 @@ static bool use_mlp_tcgen05(const dp_sim* s) {
     return s->mlp_tensor == 1 || (s->mlp_tensor == 0 && s->n >= 65536);
 }
 
+// Lanes per particle of the mma.sync pass: up to 8, until its warps fill the GPU
+// (two 256-thread CTAs on each of 152 SMs).
+static int mlp_split(const dp_sim* s) {
+    int split = 1;
+    while (split < 8 && s->n * split < 152LL * 2 * 256) split *= 2;
+    return split;
+}
+
 // Fixed-point force sums of the surrogate pass (allocated outside any graph
 // capture: run() calls this before capturing).
 static int ensure_mlp_fx(dp_sim* s) {
@@ -2387,6 +2467,13 @@ static int ensure_mlp_fx(dp_sim* s) {
     RET(dalloc_t(&s->mlp_fx, (size_t)s->n * s->dim));
     CK(cudaMemsetAsync(s->mlp_fx, 0, (size_t)s->n * s->dim * sizeof(unsigned long long), s->stream));
     return DP_OK;
+}
+
+// Lanes per particle of the force, energy, virial and Laplacian sums over lists
+// of slots (not the surrogate program's): the thresholds of the fused step.
+static int sum_lanes(const dp_sim* s) {
+    if (s->precision == DP_PREC_MLP) return mlp_split(s);
+    return s->n <= s->warp_step_max ? 32 : (s->n <= s->quad_step_max ? 4 : 1);
 }
 
 // A brick kernel: one CTA per brick, its region in dynamic shared memory.
@@ -2422,7 +2509,9 @@ static int launch_pair(dp_sim* s, cudaKernel_t k, double* out, long long* launch
                             : (km == s->lib.energy_mlp ? s->lib.energy_mlp_tc : s->lib.virial_mlp_tc);
             CK(cudaLaunchKernel((const void*)kt, dim3(grid_for(s->n, 128)), dim3(128), args, 0, s->stream));
         } else {
-            CK(cudaLaunchKernel((const void*)km, dim3(grid_for(s->n, kBlock)), dim3(kBlock), args, 0, s->stream));
+            a.mlp_split = mlp_split(s);
+            CK(cudaLaunchKernel((const void*)km, dim3(grid_for(s->n * a.mlp_split, kBlock)), dim3(kBlock), args, 0,
+                                s->stream));
         }
         if (fx) {
             void* fargs[] = {&a, &fx};
@@ -2447,7 +2536,10 @@ static int launch_pair(dp_sim* s, cudaKernel_t k, double* out, long long* launch
         RET(launch_brick(s, kb, kBlock, args));
     } else {
         void* args[] = {&a};
-        CK(cudaLaunchKernel((const void*)k, dim3(grid_for(s->n, kBlock)), dim3(kBlock), args, 0, s->stream));
+        const int lanes = sum_lanes(s);
+        if (lanes > 1)
+            k = s->lib.split[lanes == 32 ? 0 : 1][k == s->lib.forces ? 0 : (k == s->lib.energy ? 1 : (k == s->lib.virial ? 2 : 3))];
+        CK(cudaLaunchKernel((const void*)k, dim3(grid_for(s->n * lanes, kBlock)), dim3(kBlock), args, 0, s->stream));
     }
     if (launches) *launches += 1;
     return DP_OK;
@@ -2700,6 +2792,16 @@ static bool use_allpairs_step(const dp_sim* s) {
     return use_fused_step(s) && s->force_method != DP_METHOD_LIST && s->lib.step_all != nullptr;
 }
 
+static int step_lanes(const dp_sim* s) {
+    return s->step_lanes ? s->step_lanes : (s->n <= s->warp_step_max ? 32 : (s->n <= s->quad_step_max ? 4 : 1));
+}
+
+// The fused steps rebuild their own lists (dp_step_lists): no rebuild kernels in
+// the graph of steps.
+static bool use_own_lists(const dp_sim* s) {
+    return use_fused_step(s) && !use_allpairs_step(s) && list_kind(s) == kListRows && step_lanes(s) == 32;
+}
+
 // The two position buffer sets change roles (host pointers only).
 static void swap_position_buffers(dp_sim* s) {
     std::swap(s->pos, s->pos_alt);
@@ -2735,9 +2837,30 @@ static int launch_step(dp_sim* s, int kind, long long step_offset, long long* la
         if (launches) *launches += 1;
         return DP_OK;
     }
-    const int lanes = s->step_lanes ? s->step_lanes
-                                    : (s->n <= s->warp_step_max ? 32 : (s->n <= s->quad_step_max ? 4 : 1));
-    if (lanes == 32 && s->lib.step_warp) {
+    const int lanes = step_lanes(s);
+    if (end_flags & DP_END_OWN_LISTS) {
+        dp_list_args l{};
+        l.nl = s->nl;
+        l.cnt = s->cnt;
+        l.pos_ref = s->pos_ref;
+        l.shadow_ref = s->shadow_ref;
+        l.cutoff = s->cutoff;
+        bracket(s, s->cutoff, &l.lo2, &l.hi2);
+        l.kcap = s->kcap;
+        // CTAs for every SM before warps for every CTA
+        const int warps = (int)std::max<long long>(1, std::min<long long>(8, s->n / 152));
+        void* largs[] = {&pa, &ia, &l};
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid_for(s->n, warps));
+        cfg.blockDim = dim3(32 * warps);
+        cfg.stream = s->stream;
+        cudaLaunchAttribute attr = {};
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        CK(cudaLaunchKernelExC(&cfg, (const void*)s->lib.step_lists, largs));
+    } else if (lanes == 32 && s->lib.step_warp) {
         // small system: one warp per particle (32 n threads)
         CK(cudaLaunchKernel((const void*)s->lib.step_warp, dim3(grid_for(s->n * 32, kBlock)), dim3(kBlock), args, 0,
                             s->stream));
@@ -2760,7 +2883,8 @@ static int launch_step(dp_sim* s, int kind, long long step_offset, long long* la
 static int record_steps(dp_sim* s, long long steps, int kind, cudaGraph_t graph, bool conditional, bool fused,
                         long long* launches, long long* rebuild_launches) {
     *rebuild_launches = 0;
-    const bool no_list = use_allpairs_step(s);
+    const bool own_lists = use_own_lists(s);
+    const bool no_list = use_allpairs_step(s) || own_lists;
     cudaGraphConditionalHandle h = 0;  // this step's rebuild node
     if (conditional && !no_list) CK(cudaGraphConditionalHandleCreate(&h, graph, 0, 0));
     for (long long t = 0; t < steps; ++t) {
@@ -2768,7 +2892,8 @@ static int record_steps(dp_sim* s, long long steps, int kind, cudaGraph_t graph,
         // step's last CTA clears it); the non-fused kernels clear it in
         // k_integrate, before the next step's list check and pair loop
         if (no_list) {
-            // no list to keep: the step reads every particle's position
+            // no list to keep (the step reads every particle's position), or the
+            // step keeps it
         } else if (conditional) {
             // the condition of step t > 0 was set by the fused step t - 1
             RET(capture_conditional_rebuild(s, graph, h, !fused || t == 0, false, launches, rebuild_launches));
@@ -2777,7 +2902,7 @@ static int record_steps(dp_sim* s, long long steps, int kind, cudaGraph_t graph,
         }
         if (fused) {
             cudaGraphConditionalHandle next = 0;
-            int flags = DP_END_CLEAR_FAR;
+            int flags = DP_END_CLEAR_FAR | (own_lists ? DP_END_OWN_LISTS : 0);
             if (conditional && !no_list && t + 1 < steps) {
                 CK(cudaGraphConditionalHandleCreate(&next, graph, 0, 0));
                 flags |= DP_END_SET_COND;
@@ -2855,7 +2980,7 @@ static int get_graph(dp_sim* s, long long steps, int kind, GraphEntry** out) {
     }
     GraphEntry g;
     int rc = DP_ERR_CUDA;
-    if (s->conditional_graphs && s->cstream) {
+    if (s->conditional_graphs && s->lib_sets_cond && s->cstream) {
         rc = build_graph(s, steps, kind, true, &g);
         // a driver without conditional nodes: the gated kernels from now on
         if (rc != DP_OK) s->conditional_graphs = false;
@@ -3320,8 +3445,9 @@ static bool brick_program(int dim, int precision, int pmode) {
 // can then follow inside graphs.
 static std::string pair_program(int dim, int precision, int pmode, bool sig_one, bool eps_one,
                                 const std::string& pot_src, bool with_batch, int step_blocks_hint = 6,
-                                bool step_sets_cond = true, int brick_blocks = 4) {
+                                bool step_sets_cond = true, int brick_blocks = 4, int lists_blocks = 4) {
     std::string src;
+    src += "#define DP_LISTS_BLOCKS " + std::to_string(lists_blocks) + "\n";
     src += std::string("#define DP_STEP_SETS_COND ") + (step_sets_cond ? "1" : "0") + "\n";
     src += "#define DP_DIM " + std::to_string(dim) + "\n";
     if (precision == DP_PREC_MLP) src += "#define DP_MLP 1\n";
@@ -3377,16 +3503,32 @@ static int step_blocks_for(int dim, int precision, int pmode) {
 // 108,000: 30.8 against 28.8).
 static int brick_blocks_for(long long n) { return n >= 200000 ? 6 : 4; }
 
+// And for the step that keeps its own lists: 2 (no spills) where its warps do
+// not fill the GPU, 4 above (2,048 LJ particles: 15.6 us a step against 20.1;
+// 4,000: 28.3 against 22.9).
+static int lists_blocks_for(long long n) { return n < 3072 ? 2 : 4; }
+
+// The pair program sets the conditions of graph nodes. Not where the steps keep
+// their lists themselves or keep none, which is every shape but the ones set by
+// hand below the sizes of dp_step_warp: the device runtime it needs slows
+// every kernel of the program in a graph.
+static bool want_cond(const dp_sim* s) {
+    return s->conditional_graphs &&
+           !(s->precision != DP_PREC_MLP && s->fused_step && s->n <= s->warp_step_max && step_lanes(s) == 32);
+}
+
 static int rebuild_pair_lib(dp_sim* s) {
     const bool sig_one = s->pmode == DP_PAIR_CONST && s->sigma == 1.0;
     const bool eps_one = s->pmode == DP_PAIR_CONST && s->epsilon == 1.0;
     const int step_blocks = s->step_blocks ? s->step_blocks : step_blocks_for(s->dim, s->precision, s->pmode);
     const std::string src =
         pair_program(s->dim, s->precision, s->pmode, sig_one, eps_one, s->pot_src, false, step_blocks,
-                     s->conditional_graphs, s->step_blocks ? s->step_blocks : brick_blocks_for(s->n));
+                     want_cond(s), s->step_blocks ? s->step_blocks : brick_blocks_for(s->n),
+                     s->step_blocks ? s->step_blocks : lists_blocks_for(s->n));
     PairLib pl;
     RET(compile_pair_lib(src, &pl));
     s->lib = pl;
+    s->lib_sets_cond = want_cond(s);
     s->lib_valid = true;
     s->version++;
     return DP_OK;
@@ -3414,10 +3556,9 @@ int dp_set_step_launch(dp_sim* s, int lanes, int blocks_per_sm) {
         s->step_lanes = lanes;
         s->version++;
     }
-    if (blocks_per_sm != s->step_blocks) {
-        s->step_blocks = blocks_per_sm;
-        if (s->have_pot) RET(rebuild_pair_lib(s));
-    }
+    const bool blocks_changed = blocks_per_sm != s->step_blocks;
+    s->step_blocks = blocks_per_sm;
+    if (s->have_pot && (blocks_changed || want_cond(s) != s->lib_sets_cond)) RET(rebuild_pair_lib(s));
     return DP_OK;
 }
 
@@ -3426,9 +3567,10 @@ int dp_get_step_launch(dp_sim* s, int* lanes, int* blocks_per_sm) {
     const bool brick = list_kind(s) == kListBrick;
     *lanes = s->step_lanes ? s->step_lanes
              : brick       ? s->brick_lanes
-                           : (s->n <= s->warp_step_max ? 32 : (s->n <= s->quad_step_max ? 4 : 1));
+                           : step_lanes(s);
     *blocks_per_sm = s->step_blocks ? s->step_blocks
                      : brick        ? brick_blocks_for(s->n)
+                     : use_own_lists(s) ? lists_blocks_for(s->n)
                                     : step_blocks_for(s->dim, s->precision, s->pmode);
     return DP_OK;
 }
@@ -3561,7 +3703,9 @@ int dp_get_neighbor_list(dp_sim* s, int32_t* out, int kmax, int32_t* max_count) 
     int32_t* dout = nullptr;
     if (e == cudaSuccess && dalloc_t(&dout, (size_t)s->n * kmax) != DP_OK) e = cudaErrorMemoryAllocation;
     if (e == cudaSuccess) {
-        k_nl_export<<<g, kBlock, 0, s->stream>>>(rows, counts, dout, s->order, s->slot_of, s->n, kmax);
+        const bool by_rows = s->nl_kind == kListRows;
+        k_nl_export<<<g, kBlock, 0, s->stream>>>(rows, counts, dout, s->order, s->slot_of, s->n,
+                                                by_rows ? 1 : s->n, by_rows ? s->kcap : 1, kmax);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)
@@ -3642,7 +3786,8 @@ static int scalar_pair(dp_sim* s, cudaKernel_t k, double* out) {
     const bool tc = s->precision == DP_PREC_MLP && use_mlp_tcgen05(s);
     const bool all = k == s->lib.energy && s->energy_method != DP_METHOD_LIST && s->lib.energy_all;
     const long long blocks = all ? grid_for(s->n * 32, kBlock)
-                                 : (list_kind(s) == kListBrick ? s->nbricks : grid_for(s->n, tc ? 128 : kBlock));
+                                 : (list_kind(s) == kListBrick ? s->nbricks
+                                                                : grid_for(tc ? s->n : s->n * sum_lanes(s), tc ? 128 : kBlock));
     RET(ensure_partial(s, blocks));
     RET(launch_pair(s, k, nullptr, nullptr));
     k_reduce<<<1, 1024, 0, s->stream>>>(s->partial, blocks, s->dsum);
@@ -3762,7 +3907,7 @@ int dp_get_stats(dp_sim* s, dp_stats* st) {
     st->cell_capacity = 0;  // cells are contiguous slot ranges: no capacity
     st->method_used = s->use_cells ? DP_NL_CELL : DP_NL_ALLPAIRS;
     st->nl_cutoff = s->cutoff;
-    st->conditional_graphs = s->conditional_graphs ? 1 : 0;
+    st->conditional_graphs = s->conditional_graphs && !use_own_lists(s) ? 1 : 0;
     return DP_OK;
 }
 

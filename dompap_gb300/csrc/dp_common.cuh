@@ -71,6 +71,9 @@ struct dp_pair_args {
     // DP_PMODE == 0: sigma, 1/sigma, epsilon, 1/sigma^2, epsilon/sigma as double-float pairs
     float ff_const[2 * DP_FF_PARAMS];
     float f32_const[4];      // DP_PMODE == 0: sigma, 1/sigma, epsilon
+    // lists of slots: entry k of slot i at nl[k nl_k + i nl_i] (column-major n, 1;
+    // rows 1, capacity where a warp shares a particle)
+    long long nl_k, nl_i;
     // bricks (brick_kernels.cuh): per brick (first slot, particles, region
     // entries, 0), the slots of its region (brick_cap per brick) and the lists
     // (8 region indices per 16-byte chunk, chunk c of slot i at [c n + i])
@@ -78,7 +81,20 @@ struct dp_pair_args {
     const int32_t* brick_slots;
     const uint4* brick_list;
     int brick_cap;
-    int pad1;
+    int mlp_split;           // surrogate (mma.sync pass): lanes per particle
+};
+
+// A list build inside the fused step (dp_step_warp): what it writes and the
+// list's cutoff.
+struct dp_list_args {
+    int32_t* nl;
+    int32_t* cnt;
+    double* pos_ref;
+    void* shadow_ref;
+    double cutoff;
+    float lo2, hi2;  // float32 r^2 brackets of the cutoff
+    int kcap;
+    int pad;
 };
 
 // Arguments of the batched-replica kernel (batch_kernels.cuh).

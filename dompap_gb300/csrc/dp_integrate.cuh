@@ -53,6 +53,9 @@ struct dp_int_args {
 // conditional rebuild node gets its condition (need_rebuild) from here.
 #define DP_END_CLEAR_FAR 1
 #define DP_END_SET_COND 2
+// The steps rebuild their own lists (dp_step_warp): the last CTA records a
+// rebuild and leaves need_rebuild for the next step.
+#define DP_END_OWN_LISTS 4
 
 // G-JF coefficients for mass m (dompap/integrator.py:29-36): a, b dt/m,
 // b/(2m), sqrt(2 alpha T dt), dt/m.
@@ -145,7 +148,8 @@ __device__ __forceinline__ bool dp_skin_old(const void* shadow_ref, const double
 // fixed point and the 32-bit shadow (its upper word). `bad` is set when a
 // coordinate is not finite.
 template <int D, int MASSMODE, bool NVE, bool WRITE64>
-__device__ __forceinline__ bool dp_integrate_one(const dp_int_args& a, long long i, const double* F, bool& bad) {
+__device__ __forceinline__ bool dp_integrate_one(const dp_int_args& a, long long i, const double* F, bool& bad,
+                                                 int ref_far) {
     const long long n = a.n;
     double c[5];
     float cf[2];
@@ -201,18 +205,21 @@ __device__ __forceinline__ bool dp_integrate_one(const dp_int_args& a, long long
     if (WRITE64) ((typename dp_fixed64_t<D>::type*)a.pos64_out)[i] = dp_fixed64_pack<D>(X);
     // the new positions are wrapped; the list's reference positions may not be
     return dp_skin_old<D>(a.shadow_ref, a.pos_ref, n, a.unit, a.box, a.thr, a.thr_lo, a.thr_hi, i, u, xs,
-                          a.st->ref_far != 0);
+                          ref_far < 0 ? a.st->ref_far != 0 : ref_far != 0);
 }
 
 // Runtime dispatch over the mass mode and the integrator (uniform branches).
+// ref_far: whether the list's reference positions were far outside the box
+// (negative: as the status says).
 template <int D, bool WRITE64>
-__device__ __forceinline__ bool dp_integrate_dispatch(const dp_int_args& a, long long i, const double* F, bool& bad) {
+__device__ __forceinline__ bool dp_integrate_dispatch(const dp_int_args& a, long long i, const double* F, bool& bad,
+                                                      int ref_far = -1) {
     if (a.nve) {
-        if (a.massmode == 0) return dp_integrate_one<D, 0, true, WRITE64>(a, i, F, bad);
-        if (a.massmode == 1) return dp_integrate_one<D, 1, true, WRITE64>(a, i, F, bad);
-        return dp_integrate_one<D, 2, true, WRITE64>(a, i, F, bad);
+        if (a.massmode == 0) return dp_integrate_one<D, 0, true, WRITE64>(a, i, F, bad, ref_far);
+        if (a.massmode == 1) return dp_integrate_one<D, 1, true, WRITE64>(a, i, F, bad, ref_far);
+        return dp_integrate_one<D, 2, true, WRITE64>(a, i, F, bad, ref_far);
     }
-    if (a.massmode == 0) return dp_integrate_one<D, 0, false, WRITE64>(a, i, F, bad);
-    if (a.massmode == 1) return dp_integrate_one<D, 1, false, WRITE64>(a, i, F, bad);
-    return dp_integrate_one<D, 2, false, WRITE64>(a, i, F, bad);
+    if (a.massmode == 0) return dp_integrate_one<D, 0, false, WRITE64>(a, i, F, bad, ref_far);
+    if (a.massmode == 1) return dp_integrate_one<D, 1, false, WRITE64>(a, i, F, bad, ref_far);
+    return dp_integrate_one<D, 2, false, WRITE64>(a, i, F, bad, ref_far);
 }

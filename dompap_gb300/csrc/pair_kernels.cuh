@@ -361,9 +361,10 @@ __device__ __forceinline__ void dp_pair_eval_f64(const dp_pair_args& a, long lon
 // ALL: no list, every other particle is a candidate partner (dompap's
 // double-loop and vectorised force and energy methods,
 // dompap/potential.py:103-160,191-250,298-324); lane `lane` takes slots
-// lane, lane + LANES, ...
+// lane, lane + LANES, ...  listed: the row's length if the caller knows it.
 template <int ACC, int LANES = 1, bool ALL = false>
-__device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long long i, double* f, int lane = 0) {
+__device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long long i, double* f, int lane = 0,
+                                                  int listed = -1) {
     constexpr int D = DP_DIM;
     const long long n = a.n;
     const shadow_t* __restrict__ sh = (const shadow_t*)a.shadow;
@@ -396,10 +397,11 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
     // as often as its busiest lane has kept neighbours, not once per listed
     // one, and the wider the window the closer the busiest lane is to the
     // average (in a liquid about 73 % of the lanes are busy with 32, 79 % with 64).
-    const int c_all = ALL ? (int)n : a.cnt[i];
+    const int c_all = ALL ? (int)n : (listed >= 0 ? listed : a.cnt[i]);
     const int c = LANES > 1 ? (c_all > lane ? (c_all - lane + LANES - 1) / LANES : 0) : c_all;
-    const int32_t* __restrict__ row = ALL ? nullptr : a.nl + i + (LANES > 1 ? (long long)lane * n : 0LL);
-    const long long entry_stride = (long long)LANES * n;
+    // (not through the read-only path: dp_step_warp may have just written the row)
+    const int32_t* row = ALL ? nullptr : a.nl + i * a.nl_i + (LANES > 1 ? lane * a.nl_k : 0LL);
+    const long long entry_stride = LANES * a.nl_k;
     constexpr int W = LANES > 1 ? 1 : DP_WINDOW / 32;  // words of a window
     for (int base = 0; base < c; base += 32 * W) {
         uint32_t kept[W];
@@ -409,7 +411,7 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
             kept[q] = 0u;
 #pragma unroll 4
             for (int t = 0; t < w; ++t) {
-                const int j = ALL ? (first + t) * LANES + lane : __ldg(row + (long long)(first + t) * entry_stride);
+                const int j = ALL ? (first + t) * LANES + lane : row[(first + t) * entry_stride];
                 if (ALL && j == i) continue;
                 // the virial and the double-loop energy are upper-triangle sums
                 // over n < m with sigma(n, m), epsilon(n, m)
@@ -437,7 +439,7 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
             if (kept[0] == 0u) break;
             const int t = __ffs(kept[0]) - 1;
             kept[0] &= kept[0] - 1;
-            const int j = ALL ? (first + t) * LANES + lane : __ldg(row + (long long)(first + t) * entry_stride);
+            const int j = ALL ? (first + t) * LANES + lane : row[(first + t) * entry_stride];
             int tj = 0;
 #if DP_PMODE == 1
             tj = __ldg(a.types + j);
@@ -521,6 +523,14 @@ __device__ __forceinline__ void dp_step_end(const dp_int_args& b, bool old) {
     if ((unsigned)(prev & 0xffffffffull) != gridDim.x - 1) return;
     b.st->ticket = 0ull;
     const bool rebuild = ((prev + mine) >> 32) != 0;
+    if (b.end_flags & DP_END_OWN_LISTS) {
+        // every other CTA has read need_rebuild and far, and finished
+        if (b.st->need_rebuild) {
+            b.st->rebuilds += 1;
+            b.st->ref_far = b.st->far;
+        }
+        b.st->need_rebuild = rebuild ? 1 : 0;
+    }
     if (b.end_flags & DP_END_CLEAR_FAR) b.st->far = 0;
 #if DP_STEP_SETS_COND
     if (b.end_flags & DP_END_SET_COND) cudaGraphSetConditional(b.next_cond, rebuild ? 1u : 0u);
@@ -552,6 +562,52 @@ extern "C" __global__ void DP_STEP_BOUNDS dp_step(dp_pair_args a, dp_int_args b)
     dp_step_end(b, old);
 }
 
+// The list of particle i (one warp): every other particle within the cutoff by
+// the test of k_nl_build_allpairs, in ascending order, one row of the list.
+// Returns its length (the capacity at most; the status records a longer one).
+__device__ __forceinline__ int dp_build_row(const dp_pair_args& a, const dp_list_args& l, long long i, int lane,
+                                            bool far) {
+    constexpr int D = DP_DIM;
+    const long long n = a.n;
+    const shadow_t* __restrict__ sh = (const shadow_t*)a.shadow;
+    const shadow_t shi = sh[i];
+    uint32_t ui[D];
+    dp_shadow_unpack<D>(shi, ui);
+    int32_t* row = l.nl + i * l.kcap;
+    int found = 0;
+#pragma unroll 2
+    for (int base = 0; base < (int)n; base += 32) {
+        const int j = base + lane;
+        bool in = false;
+        if (j < (int)n && j != (int)i) {
+            uint32_t uj[D];
+            dp_shadow_unpack<D>(__ldg(sh + j), uj);
+            float df[D];
+            const float q = dp_shadow_q<D>(ui, uj, a.unit, df);
+            in = q <= l.hi2;
+            if (in && (far || !(q < l.lo2))) {
+                double d[D];
+#pragma unroll
+                for (int k = 0; k < D; ++k) d[k] = dp_min_image(a.pos[k * n + i] - a.pos[k * n + j], a.box[k]);
+                in = sqrt(dp_sqsum_exact<D>(d)) < l.cutoff;
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        const int at = found + __popc(m & ((1u << lane) - 1u));
+        if (in && at < l.kcap) row[at] = j;
+        found += __popc(m);
+    }
+    const int kept = min(found, l.kcap);
+    if (lane == 0) {
+        l.cnt[i] = kept;
+        ((shadow_t*)l.shadow_ref)[i] = shi;
+        atomicMax(&a.status->max_neighbors, found);
+    }
+    if (lane < D) l.pos_ref[lane * n + i] = a.pos[lane * n + i];
+    __syncwarp();
+    return kept;
+}
+
 // The fused step for small systems: LANES lanes per particle. The lanes
 // split the particle's list (dp_particle_sum<..., LANES>), their partial
 // forces are added across the group in a fixed order, and the group's first
@@ -559,7 +615,7 @@ extern "C" __global__ void DP_STEP_BOUNDS dp_step(dp_pair_args a, dp_int_args b)
 // pair loops over LANES times more threads than dp_step, whose one thread per
 // particle leaves most SMs idle.
 template <int LANES, bool ALL = false>
-__device__ __forceinline__ void dp_step_split(const dp_pair_args& a, const dp_int_args& b) {
+__device__ __forceinline__ void dp_step_split(const dp_pair_args& a, const dp_int_args& b, const dp_list_args* own) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long i = t / LANES;
     const int lane = (int)(t % LANES);
@@ -568,7 +624,12 @@ __device__ __forceinline__ void dp_step_split(const dp_pair_args& a, const dp_in
     double f[DP_DIM];
 #pragma unroll
     for (int k = 0; k < DP_DIM; ++k) f[k] = 0.0;
-    if (active) dp_particle_sum<DP_ACC_FORCE, LANES, ALL>(a, i, f, lane);
+    int listed = -1, ref_far = -1;
+    if (own && a.status->need_rebuild) {  // uniform over the grid: dp_step_end writes it
+        ref_far = a.status->far != 0;
+        if (active) listed = dp_build_row(a, *own, i, lane, ref_far != 0);
+    }
+    if (active) dp_particle_sum<DP_ACC_FORCE, LANES, ALL>(a, i, f, lane, listed);
     // every lane of the warp takes part in the shuffles (groups past the
     // last particle add zeros)
 #pragma unroll
@@ -579,19 +640,43 @@ __device__ __forceinline__ void dp_step_split(const dp_pair_args& a, const dp_in
     if (active && lane == 0) {
 #pragma unroll
         for (int k = 0; k < DP_DIM; ++k) bad = bad || !dp_isfinite_bits(f[k]);
-        old = dp_integrate_dispatch<DP_DIM, DP_FF != 0>(b, i, f, bad);
+        old = dp_integrate_dispatch<DP_DIM, DP_FF != 0>(b, i, f, bad, ref_far);
     }
     const bool any_old = __any_sync(0xffffffffu, old);
     const bool any_bad = __any_sync(0xffffffffu, bad);
     if ((threadIdx.x & 31) == 0) {
-        if (any_old) atomicExch(&b.st->need_rebuild, 1);
+        if (any_old && !own) atomicExch(&b.st->need_rebuild, 1);
         if (any_bad) atomicExch(&b.st->nonfinite, 1);
     }
     dp_step_end(b, old);
 }
 
-extern "C" __global__ void DP_STEP_BOUNDS dp_step_warp(dp_pair_args a, dp_int_args b) { dp_step_split<32>(a, b); }
-extern "C" __global__ void DP_STEP_BOUNDS dp_step_quad(dp_pair_args a, dp_int_args b) { dp_step_split<4>(a, b); }
+extern "C" __global__ void DP_STEP_BOUNDS dp_step_warp(dp_pair_args a, dp_int_args b) {
+    dp_step_split<32>(a, b, nullptr);
+}
+extern "C" __global__ void DP_STEP_BOUNDS dp_step_quad(dp_pair_args a, dp_int_args b) {
+    dp_step_split<4>(a, b, nullptr);
+}
+
+// One warp per particle, which also rebuilds the particle's list when the step
+// before asked for it (and reads need_rebuild, which no CTA writes before all
+// have read it). A row depends on this step's positions alone, so the rebuild
+// needs no kernel of its own and the graph of steps no conditional nodes, whose
+// device runtime costs every kernel of the program ~6 us in a graph; the
+// next step is placed while this one drains (programmatic dependent launch).
+// All pairs are tested, 32 a round: 500 particles take ~5 us, 8,192
+// 136 us, once in ~14 steps. Bound by the latency of its chain (gathers, pair
+// terms, the sum over the warp, the float64 integrator) and by instruction
+// fetch. LJ, float64, a step of a run before and now: 500 particles 23.2 -> 11.9
+// us, 2,048 15.6, 4,000 60 -> 22.9, 8,112 41.
+#ifndef DP_LISTS_BLOCKS
+#define DP_LISTS_BLOCKS 4
+#endif
+extern "C" __global__ void __launch_bounds__(256, DP_LISTS_BLOCKS) dp_step_lists(dp_pair_args a, dp_int_args b, dp_list_args l) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    dp_step_split<32>(a, b, &l);
+}
 
 // ---------------------------------------------------------------------------
 // No neighbour list: dompap's double-loop and vectorised methods
@@ -600,7 +685,9 @@ extern "C" __global__ void DP_STEP_BOUNDS dp_step_quad(dp_pair_args a, dp_int_ar
 // particle is a candidate, tested with the same pre-filter and pair arithmetic
 // as the list kernels), and the partial sums are added across the warp in a
 // fixed order.
-extern "C" __global__ void DP_STEP_BOUNDS dp_step_all(dp_pair_args a, dp_int_args b) { dp_step_split<32, true>(a, b); }
+extern "C" __global__ void DP_STEP_BOUNDS dp_step_all(dp_pair_args a, dp_int_args b) {
+    dp_step_split<32, true>(a, b, nullptr);
+}
 
 extern "C" __global__ void __launch_bounds__(256) dp_forces_all(dp_pair_args a) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -636,6 +723,71 @@ extern "C" __global__ void __launch_bounds__(256) dp_energy_all(dp_pair_args a) 
     v = dp_block_sum(v, smem);
     if (threadIdx.x == 0) a.partial[blockIdx.x] = v;
 }
+#endif
+
+// The same sums with LANES lanes per particle (32 up to 8,192 particles, 4 up to
+// 65,536): one thread per particle leaves most SMs idle there.
+// Forces of LJ particles in float64, before and now: 500 49 -> 8.3 us, 4,000 53 ->
+// 16.4.
+template <int LANES>
+__device__ __forceinline__ void dp_forces_split(const dp_pair_args& a) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = t / LANES;
+    const int lane = (int)(t % LANES);
+    const bool active = i < a.n;
+    double f[DP_DIM];
+#pragma unroll
+    for (int k = 0; k < DP_DIM; ++k) f[k] = 0.0;
+    if (active) dp_particle_sum<DP_ACC_FORCE, LANES>(a, i, f, lane);
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) {
+#pragma unroll
+        for (int k = 0; k < DP_DIM; ++k) f[k] += __shfl_down_sync(0xffffffffu, f[k], off, LANES);
+    }
+    if (!active || lane != 0) return;
+    bool finite = true;
+#pragma unroll
+    for (int k = 0; k < DP_DIM; ++k) {
+        a.out[k * a.n + i] = f[k];
+        finite = finite && dp_isfinite_bits(f[k]);
+    }
+    if (!finite) atomicExch(&a.status->nonfinite, 1);
+}
+
+template <int ACC, int LANES>
+__device__ __forceinline__ void dp_scalar_split(const dp_pair_args& a) {
+    __shared__ double smem[32];
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = t / LANES;
+    double v = 0.0;
+    if (i < a.n) v = dp_particle_sum<ACC, LANES>(a, i, nullptr, (int)(t % LANES));
+    v = dp_block_sum(v, smem);
+    if (threadIdx.x == 0) a.partial[blockIdx.x] = v;
+}
+
+template <int LANES>
+__device__ __forceinline__ void dp_laplacian_split(const dp_pair_args& a) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = t / LANES;
+    double v = 0.0;
+    if (i < a.n) v = dp_particle_sum<DP_ACC_LAPLACE, LANES>(a, i, nullptr, (int)(t % LANES));
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off, LANES);
+    if (i < a.n && t % LANES == 0) a.out[i] = v;
+}
+
+#if !DP_MLP
+#define DP_SPLIT_KERNELS(NAME, LANES)                                                                              \
+    extern "C" __global__ void DP_FORCES_BOUNDS dp_forces_##NAME(dp_pair_args a) { dp_forces_split<LANES>(a); }     \
+    extern "C" __global__ void DP_FORCES_BOUNDS dp_energy_##NAME(dp_pair_args a) {                                  \
+        dp_scalar_split<DP_ACC_ENERGY, LANES>(a);                                                                   \
+    }                                                                                                               \
+    extern "C" __global__ void DP_FORCES_BOUNDS dp_virial_##NAME(dp_pair_args a) {                                  \
+        dp_scalar_split<DP_ACC_VIRIAL, LANES>(a);                                                                   \
+    }                                                                                                               \
+    extern "C" __global__ void DP_FORCES_BOUNDS dp_laplacian_##NAME(dp_pair_args a) { dp_laplacian_split<LANES>(a); }
+DP_SPLIT_KERNELS(warp, 32)
+DP_SPLIT_KERNELS(quad, 4)
 #endif
 
 // Per-block partial sums of a scalar pair quantity (energy or virial); the
@@ -714,6 +866,11 @@ __device__ __forceinline__ void dp_mlp_fx_add(unsigned long long* p, float v, bo
     atomicAdd(p, (unsigned long long)dp_f2fx32(c));
 }
 
+//
+// a.mlp_split lanes share a particle (each takes every mlp_split-th entry of its
+// list): a warp holds 32 / mlp_split particles, so that a small system still fills
+// the GPU and its longest list takes that many fewer rounds. The rounds are
+// bound by latency: 4,000 particles take 39 us with 8 lanes, 203 with one.
 template <int ACC>
 __device__ __forceinline__ void dp_mlp_pass(const dp_pair_args& a, const dp_mlp_dev* mg, unsigned long long* fx) {
     constexpr int D = DP_DIM;
@@ -723,7 +880,8 @@ __device__ __forceinline__ void dp_mlp_pass(const dp_pair_args& a, const dp_mlp_
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2;
     const long long n = a.n;
-    const long long i = ((long long)blockIdx.x * (blockDim.x >> 5) + warp) * 32 + lane;
+    const int split = a.mlp_split;  // 1, 2, 4 or 8
+    const long long i = (((long long)blockIdx.x * (blockDim.x >> 5) + warp) * 32 + lane) / split;
     const bool active = i < n;
     const shadow_t* __restrict__ sh = (const shadow_t*)a.shadow;
     uint32_t ui[D];
@@ -735,7 +893,7 @@ __device__ __forceinline__ void dp_mlp_pass(const dp_pair_args& a, const dp_mlp_
     for (int k = 0; k < D; ++k) f[k] = 0.0f;
     double acc = 0.0;
     bool bad = false;
-    int kk = 0;
+    int kk = lane % split;
     while (true) {
         // this lane's next unique pair inside r_cut
         bool valid = false;
@@ -743,7 +901,7 @@ __device__ __forceinline__ void dp_mlp_pass(const dp_pair_args& a, const dp_mlp_
         float q = m.x_mean, df[D];
         while (kk < c && !valid) {
             j = __ldg(a.nl + (long long)kk * n + i);
-            ++kk;
+            kk += split;
             if (!dp_owns_pair(i, j)) continue;
             uint32_t uj[D];
             dp_shadow_unpack<D>(__ldg(sh + j), uj);
@@ -790,7 +948,11 @@ __device__ __forceinline__ void dp_mlp_pass(const dp_pair_args& a, const dp_mlp_
         }
     }
     if (ACC == DP_ACC_FORCE) {
-        if (active) {
+        for (int o = 1; o < split; o <<= 1) {
+#pragma unroll
+            for (int k = 0; k < D; ++k) f[k] += __shfl_xor_sync(0xffffffffu, f[k], o);
+        }
+        if (active && lane % split == 0) {
 #pragma unroll
             for (int k = 0; k < D; ++k) dp_mlp_fx_add(fx + (long long)k * n + i, f[k], bad);
         }

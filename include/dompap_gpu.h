@@ -60,7 +60,8 @@ typedef struct dp_stats {
     double nl_cutoff;           /* largest sigma * r_cut + skin                       */
     int32_t conditional_graphs; /* 1: run() skips the rebuild kernels on steps that need
                                    no rebuild (conditional graph nodes); 0: they are
-                                   launched every step and return at once            */
+                                   launched every step and return at once, or (up to
+                                   8,192 particles) the step kernel rebuilds itself  */
     int32_t pad;
 } dp_stats;
 
