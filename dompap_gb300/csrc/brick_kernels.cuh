@@ -147,6 +147,7 @@ __device__ __forceinline__ void dp_brick_forces(const dp_pair_args& a, const dp_
 
 template <int LANES>
 __device__ __forceinline__ void dp_step_bricks(const dp_pair_args& a, const dp_int_args& g) {
+    if (dp_step_idle(g)) return;
     const dp_brick b = dp_brick_load(a);
     bool old = false, bad = false;
     dp_brick_forces<LANES>(a, b, [&](int i, const double* f) {
@@ -154,12 +155,7 @@ __device__ __forceinline__ void dp_step_bricks(const dp_pair_args& a, const dp_i
         for (int k = 0; k < DP_DIM; ++k) bad = bad || !dp_isfinite_bits(f[k]);
         old = dp_integrate_dispatch<DP_DIM, false>(g, i, f, bad) || old;
     });
-    const bool any_old = __any_sync(0xffffffffu, old);
-    const bool any_bad = __any_sync(0xffffffffu, bad);
-    if ((threadIdx.x & 31) == 0) {
-        if (any_old) atomicExch(&g.st->need_rebuild, 1);
-        if (any_bad) atomicExch(&g.st->nonfinite, 1);
-    }
+    dp_step_flags(g, old, bad);
     dp_step_end(g, old);
 }
 

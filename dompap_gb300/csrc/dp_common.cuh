@@ -27,12 +27,14 @@ struct dp_dev_status {
     int32_t far;              // some coordinate lies outside [-L/4, 5L/4) (not yet wrapped)
     int32_t device_error;     // a bounded device-side wait gave up: the launch's results are invalid
     int32_t ref_far;          // `far` held when the current list was built (its reference positions)
-    int32_t pad;
+    int32_t parity;           // grouped steps: 1 while the second set of position buffers is current
     int64_t rebuilds;         // neighbour-list builds done on the device
     int64_t step;             // steps integrated (the RNG counter)
     // fused step in a graph: CTAs finished (low 32 bits) and CTAs with a
     // particle beyond skin/2 (high 32 bits); its last CTA resets it
     unsigned long long ticket;
+    int32_t left;             // grouped steps: still to be done by this launch
+    int32_t groups;           // grouped steps: groups run by this launch
 };
 
 // Arguments of the NVRTC-compiled pair kernels (pair_kernels.cuh); the host

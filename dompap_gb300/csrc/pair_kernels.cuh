@@ -498,22 +498,12 @@ extern "C" __global__ void DP_FORCES_BOUNDS dp_forces(dp_pair_args a) {
 #define DP_STEP_MIN_BLOCKS 0
 #endif
 
-#ifndef DP_STEP_SETS_COND
-#define DP_STEP_SETS_COND 1
-#endif
-#if DP_STEP_SETS_COND
-// Device-side condition of a graph's conditional node (CUDA device runtime).
-extern "C" __device__ void cudaGraphSetConditional(unsigned long long handle, unsigned int value);
-#endif
-
 // End of a fused step in a graph. Each CTA adds 1 and, in the upper word, 1
 // if one of its particles moved beyond skin/2, to one 64-bit counter; the
 // CTA that brings the count to the grid size is the last one: every other CTA
-// has finished (and read `far`), so it clears `far` (all positions are
-// wrapped now) and sets the condition of the next step's rebuild node from
-// the summed flags, so that node needs no condition kernel of its own. No
-// fence is needed: the condition comes from the counter itself. Called by
-// every thread of the CTA with its own `old`.
+// has finished (and read the status words), so it does the step's DP_END_*
+// work. No fence is needed: whether a rebuild is due comes from the counter
+// itself. Called by every thread of the CTA with its own `old`.
 __device__ __forceinline__ void dp_step_end(const dp_int_args& b, bool old) {
     if (b.end_flags == 0) return;  // uniform: launches outside graphs
     const int cta_old = __syncthreads_or(old ? 1 : 0);
@@ -531,12 +521,29 @@ __device__ __forceinline__ void dp_step_end(const dp_int_args& b, bool old) {
         }
         b.st->need_rebuild = rebuild ? 1 : 0;
     }
+    if (b.end_flags & DP_END_GROUP) {
+        b.st->need_rebuild = rebuild ? 1 : 0;
+        b.st->left -= 1;
+        b.st->step += 1;
+        b.st->parity ^= 1;
+    }
     if (b.end_flags & DP_END_CLEAR_FAR) b.st->far = 0;
-#if DP_STEP_SETS_COND
-    if (b.end_flags & DP_END_SET_COND) cudaGraphSetConditional(b.next_cond, rebuild ? 1u : 0u);
-#else
-    (void)rebuild;
-#endif
+}
+
+// A grouped step that has nothing to do (uniform over the grid).
+__device__ __forceinline__ bool dp_step_idle(const dp_int_args& b) {
+    return (b.end_flags & DP_END_GROUP) && (b.st->need_rebuild || b.st->left <= 0);
+}
+
+// Moved beyond skin/2: outside graphs and in graphs with a rebuild node per step
+// the flag is set at once, otherwise dp_step_end sets it.
+__device__ __forceinline__ void dp_step_flags(const dp_int_args& b, bool old, bool bad) {
+    const bool any_old = __any_sync(0xffffffffu, old);
+    const bool any_bad = __any_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0) {
+        if (any_old && !(b.end_flags & (DP_END_OWN_LISTS | DP_END_GROUP))) atomicExch(&b.st->need_rebuild, 1);
+        if (any_bad) atomicExch(&b.st->nonfinite, 1);
+    }
 }
 #if DP_STEP_MIN_BLOCKS > 0
 #define DP_STEP_BOUNDS __launch_bounds__(256, DP_STEP_MIN_BLOCKS)
@@ -544,6 +551,7 @@ __device__ __forceinline__ void dp_step_end(const dp_int_args& b, bool old) {
 #define DP_STEP_BOUNDS __launch_bounds__(256)
 #endif
 extern "C" __global__ void DP_STEP_BOUNDS dp_step(dp_pair_args a, dp_int_args b) {
+    if (dp_step_idle(b)) return;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     bool old = false, bad = false;
     if (i < a.n) {
@@ -553,12 +561,7 @@ extern "C" __global__ void DP_STEP_BOUNDS dp_step(dp_pair_args a, dp_int_args b)
         for (int k = 0; k < DP_DIM; ++k) bad = bad || !dp_isfinite_bits(f[k]);
         old = dp_integrate_dispatch<DP_DIM, DP_FF != 0>(b, i, f, bad);
     }
-    const bool any_old = __any_sync(0xffffffffu, old);
-    const bool any_bad = __any_sync(0xffffffffu, bad);
-    if ((threadIdx.x & 31) == 0) {
-        if (any_old) atomicExch(&b.st->need_rebuild, 1);
-        if (any_bad) atomicExch(&b.st->nonfinite, 1);
-    }
+    dp_step_flags(b, old, bad);
     dp_step_end(b, old);
 }
 
@@ -642,27 +645,23 @@ __device__ __forceinline__ void dp_step_split(const dp_pair_args& a, const dp_in
         for (int k = 0; k < DP_DIM; ++k) bad = bad || !dp_isfinite_bits(f[k]);
         old = dp_integrate_dispatch<DP_DIM, DP_FF != 0>(b, i, f, bad, ref_far);
     }
-    const bool any_old = __any_sync(0xffffffffu, old);
-    const bool any_bad = __any_sync(0xffffffffu, bad);
-    if ((threadIdx.x & 31) == 0) {
-        if (any_old && !own) atomicExch(&b.st->need_rebuild, 1);
-        if (any_bad) atomicExch(&b.st->nonfinite, 1);
-    }
+    dp_step_flags(b, old, bad);
     dp_step_end(b, old);
 }
 
 extern "C" __global__ void DP_STEP_BOUNDS dp_step_warp(dp_pair_args a, dp_int_args b) {
+    if (dp_step_idle(b)) return;
     dp_step_split<32>(a, b, nullptr);
 }
 extern "C" __global__ void DP_STEP_BOUNDS dp_step_quad(dp_pair_args a, dp_int_args b) {
+    if (dp_step_idle(b)) return;
     dp_step_split<4>(a, b, nullptr);
 }
 
 // One warp per particle, which also rebuilds the particle's list when the step
 // before asked for it (and reads need_rebuild, which no CTA writes before all
 // have read it). A row depends on this step's positions alone, so the rebuild
-// needs no kernel of its own and the graph of steps no conditional nodes, whose
-// device runtime costs every kernel of the program ~6 us in a graph; the
+// needs no kernel of its own and the graph of steps no conditional nodes; the
 // next step is placed while this one drains (programmatic dependent launch).
 // All pairs are tested, 32 a round: 500 particles take ~5 us, 8,192
 // 136 us, once in ~14 steps. Bound by the latency of its chain (gathers, pair
