@@ -3670,7 +3670,6 @@ int dp_get_step_launch(dp_sim* s, int* lanes, int* blocks_per_sm) {
                            : step_lanes(s);
     *blocks_per_sm = s->step_blocks ? s->step_blocks
                      : brick        ? brick_blocks_for(s->n)
-                     : use_own_lists(s) ? lists_blocks_for(s->n)
                                     : step_blocks_for(s->dim, s->precision, s->pmode);
     return DP_OK;
 }
