@@ -1894,6 +1894,7 @@ struct dp_sim {
     double* bk_mass = nullptr;
     bool nl_config_dirty = true;
     bool nl_built = false;
+    bool nl_checked = false;  // the list is known to be valid for the current positions
 
     // integrator
     double dt = 0.01, temperature = 1.0, tau = 0.1;
@@ -1974,7 +1975,9 @@ static void bracket(const dp_sim* s, double r, float* lo2, float* hi2) {
     *hi2 = std::isfinite(hi) ? (float)(hi * hi) * (1.0f + 1e-6f) : INFINITY;
 }
 
+// After every write of positions or box from outside a step.
 static int launch_shadow(dp_sim* s) {
+    s->nl_checked = false;
     ShadowArgs a{};
     a.pos = s->pos;
     a.shadow = s->shadow;
@@ -2692,8 +2695,14 @@ static int check_device_error(dp_sim* s) {
                                 "results are discarded");
 }
 
-static int write_status(dp_sim* s) {
+// Without a wait: hstat must not change before the next read_status.
+static int send_status(dp_sim* s) {
     CK(cudaMemcpyAsync(s->dstat, s->hstat, sizeof(dp_dev_status), cudaMemcpyHostToDevice, s->stream));
+    return DP_OK;
+}
+
+static int write_status(dp_sim* s) {
+    RET(send_status(s));
     CK(cudaStreamSynchronize(s->stream));
     return DP_OK;
 }
@@ -2736,33 +2745,30 @@ static int grow_after_overflow(dp_sim* s, bool* grown) {
 }
 
 // Rebuild now if needed (check) or unconditionally; handles overflow growth.
+// Two waits on the GPU when a rebuild is due and one when none is; none where
+// nothing has moved since the last check (nl_checked: cleared by everything that
+// writes positions or the box). hstat is current afterwards either way.
 static int update_nl(dp_sim* s, bool check, int* rebuilt) {
     RET(configure_nl(s));
+    if (rebuilt) *rebuilt = 0;
+    const bool usable = s->nl_built && s->nl_kind == list_kind(s);
+    if (check && usable && s->nl_checked) return DP_OK;
     if (s->use_cells) RET(ensure_perm_extras(s));
+    if (check && usable) RET(launch_skin_check(s));
     RET(read_status(s));
     const long long before = s->hstat->rebuilds;
-    if (!s->nl_built || !check || s->nl_kind != list_kind(s)) {
+    bool due = !check || !usable || s->hstat->need_rebuild != 0;
+    for (int attempt = 0; due && attempt < 8; ++attempt) {
         s->hstat->need_rebuild = 1;
-        RET(write_status(s));
-    } else {
-        RET(launch_skin_check(s));
-    }
-    for (int attempt = 0; attempt < 8; ++attempt) {
-        RET(read_status(s));
-        const bool was_needed = s->hstat->need_rebuild != 0;
-        if (!was_needed) break;
         s->hstat->max_neighbors = 0;
         s->hstat->cell_overflow = 0;
-        RET(write_status(s));
+        RET(send_status(s));
         RET(launch_rebuild(s, nullptr));
         RET(read_status(s));
-        bool grown = false;
-        RET(grow_after_overflow(s, &grown));
-        if (!grown) break;
-        s->hstat->need_rebuild = 1;
-        RET(write_status(s));
+        RET(grow_after_overflow(s, &due));
     }
     s->nl_built = true;
+    s->nl_checked = true;
     s->nl_kind = list_kind(s);
     if (rebuilt) *rebuilt = (s->hstat->rebuilds != before) ? 1 : 0;
     return DP_OK;
@@ -3159,6 +3165,7 @@ static int run_impl(dp_sim* s, long long steps, int kind, float* ms) {
     if (steps < 0) return fail(DP_ERR_ARG, "steps must be >= 0");
     // make the list current (the reference checks it at the start of every step)
     RET(update_nl(s, true, nullptr));
+    if (steps > 0) s->nl_checked = false;
     RET(ensure_partial(s, grid_for(s->n, kBlock)));
     if (s->precision == DP_PREC_MLP) RET(ensure_mlp_fx(s));
     s->launches_last = 0;
@@ -3426,6 +3433,7 @@ static int upload_i32(dp_sim* s, const int32_t* host, int32_t* dev_soa, int comp
 
 int dp_set_positions(dp_sim* s, const double* p) {
     if (!s) return fail(DP_ERR_ARG, "null handle");
+    s->nl_checked = false;
     RET(upload_aos_f64_async(s, p, s->pos));
     if (s->have_box) RET(launch_shadow(s));
     CK(cudaStreamSynchronize(s->stream));
@@ -3867,14 +3875,19 @@ int dp_run_host(dp_sim* s, const double* positions, const double* velocities, co
 int dp_forces(dp_sim* s, double* forces) {
     RET(require_ready(s));
     RET(update_nl(s, true, nullptr));
+    if (!forces) return fail(DP_ERR_ARG, "null array");
     RET(launch_pair(s, s->lib.forces, s->force, nullptr));
+    if (s->precision == DP_PREC_MLP) {  // results of a wait that gave up are not handed over
+        RET(read_status(s));
+        RET(check_device_error(s));
+    }
+    RET(download_aos_f64_async(s, s->force, forces));
     RET(read_status(s));
-    RET(check_device_error(s));
     if (s->hstat->nonfinite) {
         s->hstat->nonfinite = 0;
         RET(write_status(s));
     }
-    return download_aos_f64(s, s->force, forces);
+    return DP_OK;
 }
 
 static int scalar_pair(dp_sim* s, cudaKernel_t k, double* out) {
@@ -4031,6 +4044,7 @@ int dp_time_kernel(dp_sim* s, int which, int reps, float* ms) {
         }
     };
     const bool moves = which == DP_KERNEL_GJF || which == DP_KERNEL_NVE || which == DP_KERNEL_STEP;
+    s->nl_checked = false;
     if (moves) RET(backup_state(s));
     RET(once());  // warm-up
     CK(cudaEventRecord(s->ev0, s->stream));
@@ -4056,6 +4070,7 @@ int dp_wrap(dp_sim* s) {
     if (!s->have_box) return fail(DP_ERR_ARG, "box not set");
     dp_int_args a;
     fill_int_args(s, a, 0);
+    s->nl_checked = false;
     const unsigned g = grid_for(s->n, kBlock);
     switch (s->dim) {
         case 2: k_wrap<2><<<g, kBlock, 0, s->stream>>>(a); break;

@@ -124,3 +124,34 @@ def test_sums_match_the_oracle(n):
     assert abs(sim.get_virial() - np.sum(fr * r) / 6) <= 1e-10 * np.sum(np.abs(fr * r))
     lap = np.sum(cr - 2 * fr / r, axis=1)
     assert np.max(np.abs(sim.get_laplacian() - lap)) <= 1e-10 * np.max(np.abs(cr).sum(axis=1))
+
+
+@pytest.mark.parametrize("n", [700, 9000])
+def test_the_list_is_checked_again_after_every_change(n):
+    """Calls that read a system skip the list check only while nothing has
+    moved: after each kind of change the forces are those of a new system."""
+    pos, vel, box = _liquid(n)
+    sim = _sim(pos, vel, box, "fp64", method="cell list")
+    rng = np.random.default_rng(4)
+
+    def shift():
+        p = np.array(sim.positions)
+        p += rng.uniform(0, 1, size=3) * box + rng.normal(0, 0.05, size=p.shape)
+        sim.positions = p - np.floor(p / np.array(sim.box_vectors)) * np.array(sim.box_vectors)
+
+    def in_place():
+        sim.positions[: n // 2, 0] += 0.4
+        sim.wrap_into_box()
+
+    changes = [shift, in_place, lambda: sim.run(40), lambda: sim.run_leap_frog(9), lambda: sim.scale_box(1.01), shift,
+               lambda: sim.set_neighbor_list(skin=0.5), lambda: sim.step(), lambda: sim.scale_box(0.995)]
+    for change in changes:
+        sim.get_forces(), sim.get_potential_energy()
+        change()
+        other = _sim(np.array(sim.positions), vel, np.array(sim.box_vectors), "fp64", skin=float(sim.neighbor_list_skin),
+                     method="cell list")
+        f, g = sim.get_forces(), other.get_forces()
+        # the same pairs, summed in the order of another list
+        assert np.max(np.abs(f - g)) <= 1e-10 * np.max(np.abs(g))
+        assert abs(sim.get_virial() - other.get_virial()) <= 1e-9 * np.sum(np.abs(g))
+        assert np.allclose(sim.get_laplacian(), other.get_laplacian(), rtol=1e-9, atol=1e-9 * np.max(np.abs(g)))
