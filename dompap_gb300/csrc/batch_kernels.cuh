@@ -55,16 +55,16 @@ __device__ __forceinline__ int dp_batch_block_scan(int* cnt, int nc, int* warp_t
     return carry;
 }
 
-// visit(q) for every binned slot q != slot of the (2 R + 1)^D cells around
-// the particle in `slot`. Cells are numbered with the last axis fastest, so the
+// range(lo, hi) for every run of consecutive binned slots in the (2 R + 1)^D cells
+// around the position up. Cells are numbered with the last axis fastest, so the
 // 2 R + 1 cells of a stencil row along it hold consecutive slots: the walk
 // takes (2 R + 1)^(D-1) rows, each one slot range (two where the row wraps
 // around the box). The stencil width is a compile-time constant, so the digits
 // of the row index are taken by multiplications, not divisions; a box has at
 // least 2 R + 1 cells per axis, so one conditional subtraction wraps a cell.
-template <int D, int R, typename Visit>
-__device__ __forceinline__ void dp_batch_stencil_cells(int slot, const uint32_t* up, const int* nc, const int* s_start,
-                                                       Visit& visit) {
+template <int D, int R, typename Range>
+__device__ __forceinline__ void dp_batch_stencil_rows(const uint32_t* up, const int* nc, const int* s_start,
+                                                      Range& range) {
     constexpr int span = 2 * R + 1;
     int rows = 1;
 #pragma unroll
@@ -89,31 +89,24 @@ __device__ __forceinline__ void dp_batch_stencil_cells(int slot, const uint32_t*
         }
         base *= nl;
         // cells a..b of the row (b < nl) or a..nl-1 and 0..b-nl
-        const int e1 = s_start[base + min(b, nl - 1) + 1];
-        for (int q = s_start[base + a]; q < e1; ++q)
-            if (q != slot) visit(q);
-        if (b >= nl) {
-            const int e2 = s_start[base + (b - nl) + 1];
-            for (int q = s_start[base]; q < e2; ++q)
-                if (q != slot) visit(q);
-        }
+        range(s_start[base + a], s_start[base + min(b, nl - 1) + 1]);
+        if (b >= nl) range(s_start[base], s_start[base + (b - nl) + 1]);
     }
 }
 
-// visit(q) for every binned slot q != slot of the (2 reach + 1)^D cells
-// around the particle in `slot` (all slots when the box has no cells). Cells
-// are at least cutoff / reach wide, so the stencil covers the cutoff sphere.
-template <int D, typename Visit>
-__device__ __forceinline__ void dp_batch_stencil(bool cells, int reach, int slot, const uint32_t* up, const int* nc,
-                                                 const int* s_start, int n, Visit& visit) {
+// The ranges of the (2 reach + 1)^D cells around a position (all slots when the
+// box has no cells). Cells are at least cutoff / reach wide, so the stencil
+// covers the cutoff sphere.
+template <int D, typename Range>
+__device__ __forceinline__ void dp_batch_stencil(bool cells, int reach, const uint32_t* up, const int* nc,
+                                                 const int* s_start, int n, Range& range) {
     if (cells) {
         if (reach == 2)
-            dp_batch_stencil_cells<D, 2>(slot, up, nc, s_start, visit);
+            dp_batch_stencil_rows<D, 2>(up, nc, s_start, range);
         else
-            dp_batch_stencil_cells<D, 1>(slot, up, nc, s_start, visit);
+            dp_batch_stencil_rows<D, 1>(up, nc, s_start, range);
     } else {
-        for (int q = 0; q < n; ++q)
-            if (q != slot) visit(q);
+        range(0, n);
     }
 }
 
@@ -174,14 +167,19 @@ __device__ __forceinline__ void dp_batch_steps(const dp_batch_args& a) {
             // generation (the host changed state or settings since) or some
             // particle moved more than skin/2 since the build
             bool build = false;
+            // (the positions go into shared memory for the list loop on the way)
             if (use_list) {
                 int moved = a.list_gen[r] != a.gen;
-                for (int p = threadIdx.x; p < n && !moved; p += THREADS) {
-                    uint32_t u[D], u0[D];
-                    dp_shadow_unpack<D>(gsh[off + p], u);
-                    dp_shadow_unpack<D>(gref[off + p], u0);
-                    float df[D];
-                    moved = dp_shadow_q<D>(u, u0, unit, df) > a.skin_thr2;
+                for (int p = threadIdx.x; p < n; p += THREADS) {
+                    const sh_t v = gsh[off + p];
+                    s_sh[p] = v;
+                    if (!moved) {
+                        uint32_t u[D], u0[D];
+                        dp_shadow_unpack<D>(v, u);
+                        dp_shadow_unpack<D>(gref[off + p], u0);
+                        float df[D];
+                        moved = dp_shadow_q<D>(u, u0, unit, df) > a.skin_thr2;
+                    }
                 }
                 build = __syncthreads_or(moved);
             }
@@ -230,17 +228,47 @@ __device__ __forceinline__ void dp_batch_steps(const dp_batch_args& a) {
                     dp_shadow_unpack<D>(s_sh[slot], up);
                     const int p = s_idx[slot];
                     int cnt = 0;
-                    auto add = [&](int q) {
-                        uint32_t uq[D];
-                        dp_shadow_unpack<D>(s_sh[q], uq);
-                        float df[D];
-                        if (dp_shadow_q<D>(up, uq, unit, df) <= a.rl2) {
-                            // 8-entry chunks: chunk c of particle p at [(c n + p) 8]
-                            if (cnt < a.kmax) nl[((long long)(cnt >> 3) * n + p) * 8 + (cnt & 7)] = s_idx[q];
-                            ++cnt;
+                    // 8-entry chunks: chunk c of particle p at [(c n + p) 8],
+                    // collected in registers, the newest entry at the top
+                    uint4* to = (uint4*)nl + p;
+                    unsigned long long w0 = 0ull, w1 = 0ull;
+                    auto store = [&]() {
+                        *to = make_uint4((uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32));
+                    };
+                    // a range 32 slots at a time: a bit per partner first, then
+                    // the partners appended, so that the appending runs as often
+                    // as the busiest lane has partners and not once per
+                    // candidate that any lane of the warp lists
+                    auto add = [&](int lo, int hi) {
+                        for (int q0 = lo; q0 < hi; q0 += 32) {
+                            const int m = min(32, hi - q0);
+                            uint32_t kept = 0u;
+#pragma unroll 4
+                            for (int e = 0; e < m; ++e) {
+                                uint32_t uq[D];
+                                dp_shadow_unpack<D>(s_sh[q0 + e], uq);
+                                float df[D];
+                                if (dp_shadow_q<D>(up, uq, unit, df) <= a.rl2) kept |= 1u << e;
+                            }
+                            if (slot >= q0 && slot < q0 + 32) kept &= ~(1u << (slot - q0));
+                            for (; kept; kept &= kept - 1) {
+                                w0 = (w0 >> 16) | (w1 << 48);
+                                w1 = (w1 >> 16) | ((unsigned long long)s_idx[q0 + __ffs(kept) - 1] << 48);
+                                if ((++cnt & 7) == 0) {
+                                    if (cnt <= a.kmax) store();
+                                    to += n;
+                                }
+                            }
                         }
                     };
-                    dp_batch_stencil<D>(cells, reach, slot, up, nc, s_start, n, add);
+                    dp_batch_stencil<D>(cells, reach, up, nc, s_start, n, add);
+                    if ((cnt & 7) != 0 && cnt < a.kmax) {
+                        for (int e = cnt & 7; e < 8; ++e) {
+                            w0 = (w0 >> 16) | (w1 << 48);
+                            w1 >>= 16;
+                        }
+                        store();
+                    }
                     overflow = overflow || cnt > a.kmax;
                     a.ncnt[off + p] = min(cnt, a.kmax);
                     gref[off + p] = s_sh[slot];
@@ -257,9 +285,6 @@ __device__ __forceinline__ void dp_batch_steps(const dp_batch_args& a) {
                     for (int p = threadIdx.x; p < n; p += THREADS) s_sh[p] = gsh[off + p];
                     __syncthreads();
                 }
-            } else if (use_list) {
-                for (int p = threadIdx.x; p < n; p += THREADS) s_sh[p] = gsh[off + p];
-                __syncthreads();
             }
             // ---- 2. forces (float32) and 3. integration (float64)
             double accU = 0.0, accW = 0.0, accK = 0.0;
@@ -271,19 +296,19 @@ __device__ __forceinline__ void dp_batch_steps(const dp_batch_args& a) {
 #pragma unroll
                 for (int k = 0; k < D; ++k) f[k] = 0.0f;
                 float eu = 0.0f, ew = 0.0f;
-                auto pair = [&](int q) {
+                auto pair = [&](int q, bool sampled) {
                     uint32_t uq[D];
                     dp_shadow_unpack<D>(s_sh[q], uq);
                     float df[D];
                     const float q2 = dp_shadow_q<D>(up, uq, unit, df);
                     if (q2 <= a.rc2) {
-                        const float rinv = rsqrtf(q2);
+                        const float rinv = dp_rsqrt_normal(q2);
                         const float rr = q2 * rinv;
                         const float sf = dp_pair_f<float>(rr, rinv);
                         const float g = sf * rinv;
 #pragma unroll
                         for (int k = 0; k < D; ++k) f[k] = fmaf(g, df[k], f[k]);
-                        if (sample) {
+                        if (sampled) {
                             eu += dp_pair_u<float>(rr, rinv);
                             ew += sf * rr;
                         }
@@ -298,21 +323,30 @@ __device__ __forceinline__ void dp_batch_steps(const dp_batch_args& a) {
                     const uint4* __restrict__ rowc = (const uint4*)nl + p;
                     const int nch = (cnt + 7) >> 3;
                     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-                    uint4 c1 = nch > 0 ? __ldg(rowc) : zero;
-                    uint4 c2 = nch > 1 ? __ldg(rowc + n) : zero;
-                    for (int ch = 0; ch < nch; ++ch) {
-                        const uint4 cur = c1;
-                        c1 = c2;
-                        c2 = ch + 2 < nch ? __ldg(rowc + (long long)(ch + 2) * n) : zero;
-                        const int m = cnt - 8 * ch;
-                        const uint32_t w[4] = {cur.x, cur.y, cur.z, cur.w};
+                    auto walk = [&](bool sampled) {
+                        uint4 c1 = nch > 0 ? __ldg(rowc) : zero;
+                        uint4 c2 = nch > 1 ? __ldg(rowc + n) : zero;
+                        for (int ch = 0; ch < nch; ++ch) {
+                            const uint4 cur = c1;
+                            c1 = c2;
+                            c2 = ch + 2 < nch ? __ldg(rowc + (long long)(ch + 2) * n) : zero;
+                            const int m = cnt - 8 * ch;
+                            const uint32_t w[4] = {cur.x, cur.y, cur.z, cur.w};
 #pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (e < m) pair((int)((w[e >> 1] >> (16 * (e & 1))) & 0xFFFFu));
-                    }
+                            for (int e = 0; e < 8; ++e)
+                                if (e < m) pair((int)((w[e >> 1] >> (16 * (e & 1))) & 0xFFFFu), sampled);
+                        }
+                    };
+                    // two copies of the loop: energy and virial cost the
+                    // steps that are not sampled nothing
+                    if (sample) walk(true); else walk(false);
                 } else {
                     p = s_idx[slot];
-                    dp_batch_stencil<D>(cells, reach, slot, up, nc, s_start, n, pair);
+                    auto all = [&](int lo, int hi) {
+                        for (int q = lo; q < hi; ++q)
+                            if (q != slot) pair(q, sample);
+                    };
+                    dp_batch_stencil<D>(cells, reach, up, nc, s_start, n, all);
                 }
                 // integrate particle i (float64)
                 const long long i = off + p;
