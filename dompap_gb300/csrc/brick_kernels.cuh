@@ -13,8 +13,7 @@
 // entries a particle in a liquid), and the list is half as long in bytes
 // (k_brick_build writes it; chunks of 8 entries, one 16-byte load each).
 //
-// LANES lanes share a particle and take its chunks in turn; the forces of
-// LANES > 1 go through shared memory so that the integrator, whose float64
+// LANES lanes (1 or 4) share a particle; the forces of LANES > 1 go through shared memory so that the integrator, whose float64
 // work would cost a warp the same for 8 active lanes as for 32, runs dense.
 // Whole steps of the LJ liquid with float32 forces, before and now: 500,000
 // particles 314 -> 164 us, 20,672 45 -> 28.
@@ -60,7 +59,8 @@ __device__ __forceinline__ int dp_brick_entry(const uint4& chunk, int e) {
     return (int)((w >> (16 * (e & 1))) & 0xFFFFu);
 }
 
-// The pair sum of slot i over the chunks lane, lane + LANES, ... of its list.
+// The pair sum of slot i: every entry of its list (LANES 1), or the entries lane,
+// lane + 4, ... (LANES 4: two of each chunk, which the four lanes load as one).
 template <int ACC, int LANES>
 __device__ __forceinline__ double dp_brick_sum(const dp_pair_args& a, const dp_brick& b, int i, double* f, int lane) {
     constexpr int D = DP_DIM;
@@ -74,30 +74,35 @@ __device__ __forceinline__ double dp_brick_sum(const dp_pair_args& a, const dp_b
     const int c = a.cnt[i];
     const int chunks = (c + 7) >> 3;
     const uint4* __restrict__ list = a.brick_list + i;
-    // the virial is an upper-triangle sum over slots (symmetric parameters)
-    auto skip = [&](int id) { return ACC == DP_ACC_VIRIAL && __ldg(b.slots + id) <= i; };
-    // One pass: the pair terms are as cheap as a second gather. Two chunks in
-    // flight ahead of the one being evaluated.
     dp_shadow_unpack<D>(((const shadow_t*)a.shadow)[i], ui);
+    // One pass: the pair terms are as cheap as a second gather.
+    auto entry = [&](int id, bool listed) {
+        const uint4 h = b.at[id];
+        const uint32_t uj[4] = {h.x, h.y, h.z, h.w};
+        float df[D];
+        const float q = dp_shadow_q<D>(ui, uj, a.unit, df);
+        // the virial is an upper-triangle sum over slots (symmetric parameters)
+        if (listed && q <= a.cut2f && !(ACC == DP_ACC_VIRIAL && __ldg(b.slots + id) <= i))
+            dp_pair_eval<ACC>(a, i, 0, ti, (int)uj[D], q, df, A);
+    };
+    // two chunks in flight ahead of the one being evaluated
     const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-    const long long stride = (long long)LANES * n;
-    list += (long long)lane * n;
-    uint4 next = lane < chunks ? __ldg(list) : none;
-    uint4 after = lane + LANES < chunks ? __ldg(list + stride) : none;
-    for (int ch = lane; ch < chunks; ch += LANES) {
+    uint4 next = chunks > 0 ? __ldg(list) : none;
+    uint4 after = chunks > 1 ? __ldg(list + n) : none;
+    for (int ch = 0; ch < chunks; ++ch) {
         const uint4 cur = next;
         next = after;
-        list += stride;
-        after = ch + 2 * LANES < chunks ? __ldg(list + stride) : none;
+        list += n;
+        after = ch + 2 < chunks ? __ldg(list + n) : none;
         const int m = c - 8 * ch;
+        if (LANES == 1) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int id = dp_brick_entry(cur, e);
-            const uint4 h = b.at[id];
-            const uint32_t uj[4] = {h.x, h.y, h.z, h.w};
-            float df[D];
-            const float q = dp_shadow_q<D>(ui, uj, a.unit, df);
-            if (e < m && q <= a.cut2f && !skip(id)) dp_pair_eval<ACC>(a, i, 0, ti, (int)uj[D], q, df, A);
+            for (int e = 0; e < 8; ++e) entry(dp_brick_entry(cur, e), e < m);
+        } else {
+            const uint32_t w0 = (lane & 2) ? cur.y : cur.x, w1 = (lane & 2) ? cur.w : cur.z;
+            const int shift = 16 * (lane & 1);
+            entry((int)((w0 >> shift) & 0xFFFFu), lane < m);
+            entry((int)((w1 >> shift) & 0xFFFFu), lane + 4 < m);
         }
     }
     return A.template finish<ACC>(f);
@@ -161,7 +166,6 @@ __device__ __forceinline__ void dp_step_bricks(const dp_pair_args& a, const dp_i
 
 #define DP_BRICK_BOUNDS __launch_bounds__(256, DP_BRICK_BLOCKS)
 extern "C" __global__ void DP_BRICK_BOUNDS dp_step_brick1(dp_pair_args a, dp_int_args b) { dp_step_bricks<1>(a, b); }
-extern "C" __global__ void DP_BRICK_BOUNDS dp_step_brick2(dp_pair_args a, dp_int_args b) { dp_step_bricks<2>(a, b); }
 extern "C" __global__ void DP_BRICK_BOUNDS dp_step_brick4(dp_pair_args a, dp_int_args b) { dp_step_bricks<4>(a, b); }
 
 extern "C" __global__ void __launch_bounds__(256) dp_forces_brick(dp_pair_args a) {

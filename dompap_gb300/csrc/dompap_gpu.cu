@@ -917,7 +917,21 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_brick_build(NlArgs a, Bric
                         if (!in) m &= ~bit;
                     }
                 }
-                // the quad's entries one lane after another
+                // lane c takes the 32 entries from t0 + 32 c, so that the row is in
+                // the order of the region (the order of k_nl_build_cells: the
+                // same float32 sums): byte c of each lane's word holds its two
+                // columns of the lane's four tiles
+                {
+                    uint32_t mixed = 0u;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        uint32_t x = (__shfl_sync(0xffffffffu, m, q, 4) >> (24 - 8 * c)) & 0xFFu;
+                        x = (x | (x << 12)) & 0x000F000Fu;
+                        x = (x | (x << 6)) & 0x03030303u;
+                        mixed |= x << (6 - 2 * q);
+                    }
+                    m = mixed;
+                }
                 const int mine = __popc(m);
                 int upto = mine;
 #pragma unroll
@@ -933,14 +947,14 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_brick_build(NlArgs a, Bric
                     for (; left > 0; --left, to += a.nl_k) {
                         const int s = __clz(m);
                         m &= ~(0x80000000u >> s);
-                        *to = rslot[t0 + 8 * (s >> 1) + 2 * c + (s & 1)];
+                        *to = rslot[t0 + 32 * c + s];
                     }
                 } else {
                     uint16_t* to = (uint16_t*)b.list + (((long long)(at >> 3) * n + i) * 8 + (at & 7));
                     for (int e = at; left > 0; --left) {
                         const int s = __clz(m);
                         m &= ~(0x80000000u >> s);
-                        *to = (uint16_t)(t0 + 8 * (s >> 1) + 2 * c + (s & 1));
+                        *to = (uint16_t)(t0 + 32 * c + s);
                         ++e;
                         to += (e & 7) ? 1 : 8 * n - 7;
                     }
@@ -1558,8 +1572,8 @@ struct PairLib {
     // no neighbour list (dompap's double-loop methods): fused step, forces, energy
     cudaKernel_t step_all = nullptr, forces_all = nullptr, energy_all = nullptr;
     // bricks of cells (not in 4-D, with dense parameters or in the surrogate
-    // program): fused step with 1, 2 or 4 lanes per particle, forces, scalars
-    cudaKernel_t step_brick[3] = {nullptr, nullptr, nullptr};
+    // program): fused step with 1 or 4 lanes per particle, forces, scalars
+    cudaKernel_t step_brick[2] = {nullptr, nullptr};
     cudaKernel_t forces_brick = nullptr, energy_brick = nullptr, virial_brick = nullptr, laplacian_brick = nullptr;
     cudaKernel_t batch[4] = {nullptr, nullptr, nullptr, nullptr};  // 128, 256, 512, 1024 threads
     cudaKernel_t forces_mlp = nullptr, energy_mlp = nullptr, virial_mlp = nullptr, mlp_finish = nullptr;
@@ -1741,8 +1755,7 @@ static int compile_pair_lib(const std::string& src, PairLib* out) {
     }
     if (src.find("#define DP_BRICKS 1") != std::string::npos) {
         CK(cudaLibraryGetKernel(&pl.step_brick[0], pl.lib, "dp_step_brick1"));
-        CK(cudaLibraryGetKernel(&pl.step_brick[1], pl.lib, "dp_step_brick2"));
-        CK(cudaLibraryGetKernel(&pl.step_brick[2], pl.lib, "dp_step_brick4"));
+        CK(cudaLibraryGetKernel(&pl.step_brick[1], pl.lib, "dp_step_brick4"));
         CK(cudaLibraryGetKernel(&pl.forces_brick, pl.lib, "dp_forces_brick"));
         CK(cudaLibraryGetKernel(&pl.energy_brick, pl.lib, "dp_energy_brick"));
         CK(cudaLibraryGetKernel(&pl.virial_brick, pl.lib, "dp_virial_brick"));
@@ -2130,12 +2143,12 @@ static int configure_bricks(dp_sim* s) {
     // The float32 pair kernels run on bricks where a particle lists 32 or more
     // (with a dozen listed, the region's copy costs more than the gathers it
     // saves: 101 against 78 us a step for 1,048,576 harmonic spheres), above the
-    // sizes of dp_step_warp. Lanes per particle: as many as fill the GPU (LJ us a
-    // step with 1 / 2 / 4: 9,464 particles 18.5 / 14.4 / 12.4; 42,592 20.5 / 18.6 /
-    // 22.6; 78,732 26.7 / 30.8 / 38.8).
+    // sizes of dp_step_warp. Lanes per particle: those of dp_step_quad and dp_step,
+    // so that the float32 sums are the same (LJ us a step with 1 / 4: 9,464 particles
+    // 18.5 / 12.4; 42,592 20.5 / 22.6; 78,732 26.7 / 38.8).
     const double sphere = s->dim == 2 ? pi * c * c : 4.0 / 3.0 * pi * c * c * c;
     s->brick_pairs = s->dim <= 3 && s->n > s->warp_step_max && (double)s->n / volume * sphere >= 32.0;
-    s->brick_lanes = s->n < 32768 ? 4 : (s->n < 65536 ? 2 : 1);
+    s->brick_lanes = s->n <= s->quad_step_max ? 4 : 1;
     s->brick_threads = std::max(64, std::min(256, ((int)(1.2 * mean * s->brick_lanes) + 31) & ~31));
     return DP_OK;
 }
@@ -2259,7 +2272,8 @@ enum { kListFull = 0, kListHalf = 1, kListBrick = 2, kListRows = 3 };
 static int list_kind(const dp_sim* s) {
     if (s->precision == DP_PREC_MLP) return kListHalf;
     if (s->brick_pairs && s->step_lanes != 32 && s->lib.forces_brick) return kListBrick;
-    return s->n <= s->warp_step_max ? kListRows : kListFull;
+    // float32 sums follow the order of the list: cell lists keep theirs
+    return s->n <= s->warp_step_max && !(s->precision == DP_PREC_FP32 && s->use_cells) ? kListRows : kListFull;
 }
 
 template <int D>
@@ -2314,7 +2328,7 @@ static int launch_rebuild(dp_sim* s, long long* launches) {
     fill_scale(s, nullptr, na.unit);
     for (int k = 0; k < DP_MAX_DIM; ++k) na.box[k] = (k < s->dim) ? s->box[k] : 1.0;
     long long nl_launches = 0;
-    if (s->n <= s->warp_step_max) {
+    if (s->n <= s->warp_step_max && list_kind(s) != kListFull) {
         const unsigned gr = grid_for(s->n * 32, kBlock);
         switch (s->dim) {
             case 2: k_nl_build_rows<2><<<gr, kBlock, 0, s->stream>>>(na); break;
@@ -2861,7 +2875,7 @@ static int launch_step(dp_sim* s, int kind, long long step_offset, long long* la
     }
     if (list_kind(s) == kListBrick) {
         const int lanes = s->step_lanes ? s->step_lanes : s->brick_lanes;
-        RET(launch_brick(s, s->lib.step_brick[lanes == 1 ? 0 : (lanes == 2 ? 1 : 2)], s->brick_threads, args));
+        RET(launch_brick(s, s->lib.step_brick[lanes == 1 ? 0 : 1], s->brick_threads, args));
         if (launches) *launches += 1;
         return DP_OK;
     }
@@ -2941,13 +2955,13 @@ static int record_steps(dp_sim* s, long long steps, int kind, cudaGraph_t graph,
     return DP_OK;
 }
 
-// Grouped steps: cell lists of more than a warp per particle.
+// Grouped steps: cell lists (the small systems that keep their own lists aside).
 constexpr int kGroupSteps = 12;  // even: a group that is not interrupted leaves the first position set current
 
 static bool use_groups(const dp_sim* s) {
     const int kind = list_kind(s);
     return s->conditional_graphs && s->cstream && s->bstream && use_fused_step(s) && !use_allpairs_step(s) &&
-           !use_own_lists(s) && s->use_cells && s->reorder && s->n > s->warp_step_max &&
+           !use_own_lists(s) && s->use_cells && s->reorder &&
            (kind == kListFull || kind == kListBrick);
 }
 
