@@ -8,13 +8,13 @@
 //  * particle state lives in HBM as SoA float64 pos/vel/beta/force[k*N + i]
 //    plus int32 images; a fixed-point copy of the positions (uint32 per axis,
 //    packed in one 8/16-byte vector per particle) feeds the pair pre-filter;
-//  * the neighbour list is column-major nl[k*N + i] with counts cnt[i];
-//  * run(steps) replays CUDA graphs of `chunk` steps. Each step is
-//    [gated rebuild: cell clear, cell fill, cell sort, Verlet build, done]
-//    -> pair forces -> integrate + wrap + skin test (sets need_rebuild).
-//    The rebuild kernels return at once unless need_rebuild is set, so the
-//    graph needs no host decision. After each chunk the host reads the status
-//    word; on a neighbour-list or cell overflow it restores the chunk's start
+//  * lists hold slots, column-major nl[k*N + i] with counts cnt[i] (in rows for
+//    systems of at most a warp per particle), or 16-bit region indices for the
+//    brick kernels;
+//  * run(steps) launches CUDA graphs of fused steps: groups of steps with one
+//    conditional rebuild each in a loop on the device, or, for small systems,
+//    steps that rebuild their own lists. After each chunk the host reads the
+//    status word; on a list or region overflow it restores the chunk's start
 //    state, grows the capacity and replays the chunk.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
