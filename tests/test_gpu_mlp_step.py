@@ -69,3 +69,21 @@ def test_training_is_reproducible_and_splits():
     la = a.train(12, batch=1000, lr0=1e-3, lr1=1e-3)
     lb = np.concatenate([b.train(5, batch=1000, lr0=1e-3, lr1=1e-3), b.train(7, batch=1000, lr0=1e-3, lr1=1e-3)])
     assert np.array_equal(a.params(), b.params()) and np.array_equal(la, lb)
+
+
+@pytest.mark.parametrize("scale", [1.0, 30.0, 1000.0])
+def test_gradient_sums_of_small_and_large_terms(scale):
+    """Terms on both sides of 2^31 fixed-point units (1/32 of a gradient, 1/2 of
+    a loss): the 32-bit and the shifted conversion, both signs."""
+    sur = _surrogate()
+    rng = np.random.default_rng(11)
+    n = 129
+    s = (rng.uniform(0.8, 3.0, n) ** 2).astype(np.float32)
+    t = (scale * rng.normal(0, 1, (n, 2))).astype(np.float32)
+    x = (s.astype(np.float64) - float(sur.norm[0])) * float(sur.norm[1])
+    loss, g = sur.gradients(s, t, wf=0.7, accurate=True)
+    loss_ref, g_ref = mlp_ref.loss_and_grad(sur.params(), x, t.astype(np.float64), wf=0.7)
+    # as at the tile edges: bf16 operands of the backward products, 2^-9 each
+    assert abs(loss - loss_ref) <= 5e-3 * loss_ref
+    for sl in (slice(0, 64), slice(64, 128), slice(128, 4224), slice(4224, 4288), slice(4288, 4416), slice(4416, 4418)):
+        assert np.linalg.norm(g[sl] - g_ref[sl]) <= 3e-2 * np.linalg.norm(g_ref[sl])
