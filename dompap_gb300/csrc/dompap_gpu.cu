@@ -1344,13 +1344,25 @@ constexpr int kRdfChunk = 64;    // particles j of one work item
 constexpr int kRdfQueue = 64;    // queued near-edge pairs per warp (a round adds at most 32)
 constexpr int kRdfItems = 65536; // items between flushes: 65536 * 256 * 64 * 2 < 2^32 counts per bin
 
+// Small systems (at most one work item per SM): a call is its launches and one
+// thread's chain of partners, so the types are compared in the kernel and not
+// selected before it, and an item has a quarter of the partners. 500 particles,
+// 200 bins: all pairs 73 -> 59 us a call, two calls with types 171 -> 137;
+// 1,372: 74 -> 60, 175 -> 139. At 2,048 with the longer items 79 -> 84 (all
+// pairs: the comparison is in the loop), hence a form of its own; from there on
+// the selected lists are as fast or faster (4,000: 199 against 215).
+constexpr int kRdfSmallItems = 152;
+constexpr int kRdfSmallChunk = 16;
+
 struct RdfArgs {
+    const int32_t* types;     // of the small form, which compares them (null: every particle)
+    int type_a, type_b;       // negative: every type
     const double* pos;
     const void* shadow;
     const double* edges;
     const int32_t* idx_a;     // slots of the particles i, j (null: every slot)
     const int32_t* idx_b;
-    const int32_t* selected;  // their numbers, [2] (null: n)
+    const int32_t* selected;  // their numbers, [2], [1] where A and B are the same set (null: n)
     unsigned long long* counts;
     long long n;
     int nbins;
@@ -1362,9 +1374,14 @@ struct RdfArgs {
     float unit[DP_MAX_DIM];
 };
 
-// Slots of the particles of one type, in no particular order (the histogram
-// does not depend on it).
-__global__ void k_rdf_select(const int32_t* __restrict__ types, long long n, int type, int32_t* idx, int32_t* count) {
+// Slots of the particles of type a (blockIdx.y = 0) and b (1), in no particular
+// order (the histogram does not depend on it). One launch for both, and none
+// for b where it is the same set: on a small system the call is its launches.
+__global__ void k_rdf_select(const int32_t* __restrict__ types, long long n, int type_a, int type_b, int32_t* idx,
+                             int32_t* count) {
+    const int type = blockIdx.y ? type_b : type_a;
+    idx += blockIdx.y * n;
+    count += blockIdx.y;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool take = i < n && (type < 0 || types[i] == type);
     const unsigned m = __ballot_sync(0xffffffffu, take);
@@ -1404,12 +1421,14 @@ __device__ __forceinline__ void rdf_exact(const RdfArgs& a, const double* edges,
     if (b >= 0) atomicAdd(hist + b, twice ? 2u : 1u);
 }
 
-template <int D>
+template <int D, bool SMALL>
 __global__ void __launch_bounds__(kBlock) k_rdf(RdfArgs a) {
+    constexpr int kChunk = SMALL ? kRdfSmallChunk : kRdfChunk;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     typedef typename dp_shadow_t<D>::type sh_t;
-    __shared__ sh_t tile[kRdfChunk];
-    __shared__ int32_t tslot[kRdfChunk];
+    __shared__ sh_t tile[kChunk];
+    __shared__ int32_t tslot[kChunk];
+    __shared__ bool tmine[SMALL ? kChunk : 1];
     __shared__ int2 queue[kBlock / 32][kRdfQueue];
     double* edges = (double*)smem_raw;                          // [nbins + 1]
     float* ef = (float*)(edges + a.nbins + 1);                  // [nbins + 1]
@@ -1439,8 +1458,8 @@ __global__ void __launch_bounds__(kBlock) k_rdf(RdfArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned int* my_hist = hist + (lane % a.copies) * nb;
     const sh_t* __restrict__ sh = (const sh_t*)a.shadow;
-    const int na = a.selected ? a.selected[0] : (int)a.n, nbp = a.selected ? a.selected[1] : (int)a.n;
-    const long long rows = (na + kBlock - 1) / kBlock, chunks = (nbp + kRdfChunk - 1) / kRdfChunk;
+    const int na = a.selected ? a.selected[0] : (int)a.n, nbp = a.symmetric ? na : (a.selected ? a.selected[1] : (int)a.n);
+    const long long rows = (na + kBlock - 1) / kBlock, chunks = (nbp + kChunk - 1) / kChunk;
     const float rmax = r1 * (1.0f + 2e-6f) + 2.0f * a.abs_tol;
     const float qmax = rmax * rmax * (1.0f + 1e-6f);
     int queued = 0;  // entries in this warp's queue (uniform)
@@ -1460,22 +1479,23 @@ __global__ void __launch_bounds__(kBlock) k_rdf(RdfArgs a) {
     for (long long w = blockIdx.x; w < rows * chunks; w += gridDim.x) {
         const long long row = w / chunks, chunk = w - row * chunks;
         // symmetric: only pairs with j >= i
-        if (a.symmetric && (chunk + 1) * kRdfChunk <= row * kBlock) continue;
+        if (a.symmetric && (chunk + 1) * kChunk <= row * kBlock) continue;
         if (++since == kRdfItems) {
             flush();
             since = 1;
         }
-        const int j0 = (int)(chunk * kRdfChunk), jn = min(kRdfChunk, nbp - j0);
+        const int j0 = (int)(chunk * kChunk), jn = min(kChunk, nbp - j0);
         __syncthreads();
         if ((int)threadIdx.x < jn) {
             const int slot = a.idx_b ? a.idx_b[j0 + threadIdx.x] : j0 + (int)threadIdx.x;
             tslot[threadIdx.x] = slot;
             tile[threadIdx.x] = sh[slot];
+            if (SMALL) tmine[threadIdx.x] = !a.types || a.type_b < 0 || a.types[slot] == a.type_b;
         }
         __syncthreads();
         const int i = (int)(row * kBlock) + threadIdx.x;
-        const bool active = i < na;
-        const int si = active ? (a.idx_a ? a.idx_a[i] : i) : 0;
+        const int si = i < na ? (a.idx_a ? a.idx_a[i] : i) : 0;
+        const bool active = i < na && (!SMALL || !a.types || a.type_a < 0 || a.types[si] == a.type_a);
         uint32_t ui[D];
         dp_shadow_unpack<D>(sh[si], ui);
         for (int t = 0; t < jn; ++t) {
@@ -1485,7 +1505,7 @@ __global__ void __launch_bounds__(kBlock) k_rdf(RdfArgs a) {
             const float q = dp_shadow_q<D>(ui, uj, a.unit, df);
             const int j = j0 + t;
             bool near = false;
-            if (active && q <= qmax && (!a.symmetric || j >= i)) {
+            if (active && q <= qmax && (!a.symmetric || j >= i) && (!SMALL || tmine[t])) {
                 const float r = q > 0.0f ? q * rsqrtf(q) : 0.0f;
                 const float tol = fmaf(1e-6f, r, a.abs_tol);
                 int b = table[max(0, min((int)((r - r0) * inv_w), a.cells - 1))];
@@ -4103,9 +4123,10 @@ int dp_rdf_counts(dp_sim* s, int type_a, int type_b, const double* edges, int nb
     if ((type_a >= 0 || type_b >= 0) && !s->have_types) return fail(DP_ERR_ARG, "particle types not set");
     for (int b = 0; b < nbins; ++b)
         if (!(edges[b] <= edges[b + 1])) return fail(DP_ERR_ARG, "r_bins array must be sorted in ascending order.");
-    // edges and counts in one buffer of the handle, grown as needed
+    // edges, the selections' lengths and counts in one buffer of the handle,
+    // grown as needed: the last two are cleared together
     if (nbins > s->rdf_bins) {
-        RET(dalloc(&s->rdf_buf, (size_t)(nbins + 1) * sizeof(double) + (size_t)nbins * sizeof(unsigned long long)));
+        RET(dalloc(&s->rdf_buf, (size_t)(nbins + 1) * sizeof(double) + (size_t)(nbins + 1) * sizeof(unsigned long long)));
         s->rdf_bins = nbins;
     }
     RdfArgs a{};
@@ -4113,7 +4134,8 @@ int dp_rdf_counts(dp_sim* s, int type_a, int type_b, const double* edges, int nb
     a.pos = s->pos;
     a.shadow = s->shadow;
     a.edges = dedges;
-    a.counts = (unsigned long long*)(dedges + s->rdf_bins + 1);
+    unsigned long long* lengths = (unsigned long long*)(dedges + s->rdf_bins + 1);
+    a.counts = lengths + 1;
     a.n = s->n;
     a.nbins = nbins;
     // two cells per bin: most need no second compare; at most 4096, so that the
@@ -4127,15 +4149,19 @@ int dp_rdf_counts(dp_sim* s, int type_a, int type_b, const double* edges, int nb
     fill_scale(s, nullptr, a.unit);
     a.abs_tol = (float)(4.0 * lmax / 4294967296.0 * std::sqrt((double)s->dim) + 1e-30);
     const unsigned gn = grid_for(s->n, kBlock);
+    const bool small = (long long)gn * ((s->n + kRdfChunk - 1) / kRdfChunk) <= kRdfSmallItems;
     CK(cudaMemcpyAsync(dedges, edges, (nbins + 1) * sizeof(double), cudaMemcpyHostToDevice, s->stream));
-    CK(cudaMemsetAsync(a.counts, 0, nbins * sizeof(unsigned long long), s->stream));
-    if (type_a >= 0 || type_b >= 0) {
-        // the two selections and their lengths in one buffer of the handle
-        if (!s->rdf_sel) RET(dalloc_t(&s->rdf_sel, 2 * (size_t)s->n + 2));
-        int32_t* len = s->rdf_sel + 2 * s->n;
-        CK(cudaMemsetAsync(len, 0, 2 * sizeof(int32_t), s->stream));
-        k_rdf_select<<<gn, kBlock, 0, s->stream>>>(s->types, s->n, type_a, s->rdf_sel, len);
-        k_rdf_select<<<gn, kBlock, 0, s->stream>>>(s->types, s->n, type_b, s->rdf_sel + s->n, len + 1);
+    CK(cudaMemsetAsync(lengths, 0, (nbins + 1) * sizeof(unsigned long long), s->stream));
+    if ((type_a >= 0 || type_b >= 0) && small) {
+        a.types = s->types;
+        a.type_a = type_a;
+        a.type_b = type_b;
+    } else if (type_a >= 0 || type_b >= 0) {
+        // the two selections in one buffer of the handle
+        if (!s->rdf_sel) RET(dalloc_t(&s->rdf_sel, 2 * (size_t)s->n));
+        int32_t* len = (int32_t*)lengths;
+        k_rdf_select<<<dim3(gn, a.symmetric ? 1 : 2), kBlock, 0, s->stream>>>(s->types, s->n, type_a, type_b,
+                                                                             s->rdf_sel, len);
         CK(cudaGetLastError());
         a.idx_a = s->rdf_sel;
         a.idx_b = a.symmetric ? s->rdf_sel : s->rdf_sel + s->n;
@@ -4143,7 +4169,8 @@ int dp_rdf_counts(dp_sim* s, int type_a, int type_b, const double* edges, int nb
     }
     const size_t smem = (size_t)(nbins + 1) * (sizeof(double) + sizeof(float)) +
                         (size_t)a.copies * nbins * sizeof(unsigned int) + (size_t)a.cells * sizeof(uint16_t);
-    const long long items = (long long)gn * ((s->n + kRdfChunk - 1) / kRdfChunk);
+    const int chunk = small ? kRdfSmallChunk : kRdfChunk;
+    const long long items = (long long)gn * ((s->n + chunk - 1) / chunk);
     const unsigned g = (unsigned)std::min<long long>(items, 152LL * 8);
     auto launch = [&](auto kernel) -> cudaError_t {
         if (smem > 32 * 1024) {
@@ -4154,7 +4181,10 @@ int dp_rdf_counts(dp_sim* s, int type_a, int type_b, const double* edges, int nb
         kernel<<<g, kBlock, smem, s->stream>>>(a);
         return cudaGetLastError();
     };
-    CK(s->dim == 2 ? launch(k_rdf<2>) : (s->dim == 3 ? launch(k_rdf<3>) : launch(k_rdf<4>)));
+    if (small)
+        CK(s->dim == 2 ? launch(k_rdf<2, true>) : (s->dim == 3 ? launch(k_rdf<3, true>) : launch(k_rdf<4, true>)));
+    else
+        CK(s->dim == 2 ? launch(k_rdf<2, false>) : (s->dim == 3 ? launch(k_rdf<3, false>) : launch(k_rdf<4, false>)));
     CK(cudaMemcpyAsync(counts, a.counts, nbins * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return DP_OK;

@@ -66,6 +66,21 @@ def test_counts_equal_np_histogram(n, dim):
             assert np.array_equal(got, _expected(pos, box, edges, *sel)), (name, a, b)
 
 
+@pytest.mark.parametrize("n", [1536, 1537, 1600])
+@pytest.mark.parametrize("dim", [2, 3, 4])
+def test_typed_counts_beside_the_line_between_the_two_forms(n, dim):
+    """Up to 152 work items (256 particles x 64 partners; 1,536 particles have
+    144, 1,537 have 175) the kernel compares the types, above they are selected."""
+    rng = np.random.default_rng([n, dim, 1])
+    box = np.array([9.0, 8.5, 10.0, 9.5])[:dim]
+    pos = rng.uniform(0.0, 1.0, size=(n, dim)) * box
+    types = rng.integers(0, 3, size=n).astype(np.int32)
+    sim = _sim(pos, box, types)
+    for a, b in ((-1, -1), (1, 1), (0, 2), (-1, 1), (1, -1), (7, 7)):
+        sel = [np.arange(n) if t < 0 else np.nonzero(types == t)[0] for t in (a, b)]
+        assert np.array_equal(_counts(sim, EDGES["uneven"], a, b), _expected(pos, box, EDGES["uneven"], *sel)), (a, b)
+
+
 def test_distances_on_bin_edges():
     """A simple cubic lattice: every distance is the square root of an integer,
     and the edges are exactly those distances."""
