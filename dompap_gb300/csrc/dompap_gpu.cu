@@ -2291,7 +2291,7 @@ static void fill_perm_args(const dp_sim* s, PermArgs& p) {
 enum { kListFull = 0, kListHalf = 1, kListBrick = 2, kListRows = 3 };
 static int list_kind(const dp_sim* s) {
     if (s->precision == DP_PREC_MLP) return kListHalf;
-    if (s->brick_pairs && s->step_lanes != 32 && s->lib.forces_brick) return kListBrick;
+    if (s->bricks && s->brick_pairs && s->step_lanes != 32 && s->lib.forces_brick) return kListBrick;
     // float32 sums follow the order of the list: cell lists keep theirs
     return s->n <= s->warp_step_max && !(s->precision == DP_PREC_FP32 && s->use_cells) ? kListRows : kListFull;
 }
@@ -2761,8 +2761,9 @@ static int grow_after_overflow(dp_sim* s, bool* grown) {
         // a denser region than expected
         const int want = ((int)(s->hstat->cell_overflow * 1.2) + 32 + 31) & ~31;
         if (want > kBrickMaxCap) {
+            // the lists become lists of slots (list_kind), the pair kernels theirs
             s->bricks_off = true;
-            s->bricks = false;
+            s->bricks = s->brick_pairs = false;
             s->version++;
         } else {
             RET(alloc_brick_slots(s, want));
