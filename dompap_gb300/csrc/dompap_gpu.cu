@@ -14,8 +14,9 @@
 //  * run(steps) launches CUDA graphs of fused steps: groups of steps with one
 //    conditional rebuild each in a loop on the device, or, for small systems,
 //    steps that rebuild their own lists. After each chunk the host reads the
-//    status word; on a list or region overflow it restores the chunk's start
-//    state, grows the capacity and replays the chunk.
+//    status word; on a list or region overflow it grows the capacity. Grouped
+//    steps have stopped at that build and go on from it; other chunks are
+//    replayed from their start state.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <nvrtc.h>
@@ -833,7 +834,7 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_brick_build(NlArgs a, Bric
         b.info[blockIdx.x] = make_int4(first, count, min(entries, b.cap), 0);
         if (entries > b.cap) atomicMax(&a.st->cell_overflow, entries);
     }
-    if (entries > b.cap) {  // uniform; the host grows the capacity and replays; until then no list
+    if (entries > b.cap) {  // uniform; no list: the host makes room and has it built again before it counts
         for (int p = threadIdx.x; p < count; p += blockDim.x) a.cnt[first + p] = 0;
         return;
     }
@@ -1124,8 +1125,12 @@ __global__ void __launch_bounds__(128) k_selftest_bounded_wait(dp_dev_status* st
     if (warp == 0) dp_tmem_dealloc(s_tmem, 64);
 }
 
-__global__ void k_rebuild_done(dp_dev_status* st) {
+// kcap, region: room of a row and of a brick's region. Grouped steps stop at a build
+// that did not fit (its lists are cut short or empty): the steps before it stand,
+// and the host makes room and goes on from there.
+__global__ void k_rebuild_done(dp_dev_status* st, int kcap, int region) {
     if (st->need_rebuild) {
+        if (st->max_neighbors > kcap || st->cell_overflow > region) st->left = 0;
         st->need_rebuild = 0;
         st->rebuilds += 1;
         st->ref_far = st->far;  // the list's reference positions are the current ones
@@ -2419,7 +2424,7 @@ static int launch_rebuild(dp_sim* s, long long* launches) {
         }
         nl_launches = 1;
     }
-    k_rebuild_done<<<1, 1, 0, s->stream>>>(s->dstat);
+    k_rebuild_done<<<1, 1, 0, s->stream>>>(s->dstat, s->kcap, s->bricks ? s->brick_cap : 0x7FFFFFFF);
     CK(cudaGetLastError());
     if (launches) *launches += nl_launches + 1;
     return DP_OK;
@@ -3208,18 +3213,18 @@ static int run_impl(dp_sim* s, long long steps, int kind, float* ms) {
     if (ms) CK(cudaEventRecord(s->ev0, s->stream));
     const long long chunk = chunk_steps(s);
     long long done = 0;
-    int retries = 0;
+    int retries = 0;  // attempts since the last step that stands
     while (done < steps) {
         const long long c = std::min(chunk, steps - done);
         const long long step0 = s->hstat->step;  // hstat is current: every path here ends in read_status
         const long long rebuilds0 = s->hstat->rebuilds;
-        // a chunk needs the backup only if a list build inside it can
-        // overflow: at a later step, or at its first step when a rebuild is
-        // pending (hstat is current here)
-        const bool backed_up = !use_allpairs_step(s) && (c > 1 || s->hstat->need_rebuild != 0);
-        if (backed_up) RET(backup_state(s));
         GraphEntry* g = nullptr;
         const bool groups = use_groups(s);
+        // a chunk needs the backup only if a list build inside it can
+        // overflow: at a later step, or at its first step when a rebuild is
+        // pending (hstat is current here); grouped steps stop there
+        const bool backed_up = !groups && !use_allpairs_step(s) && (c > 1 || s->hstat->need_rebuild != 0);
+        if (backed_up) RET(backup_state(s));
         RET(get_graph(s, groups ? -1 : c, kind, &g));
         if (groups) {
             k_group_start<<<1, 1, 0, s->stream>>>(s->dstat, (int)c);
@@ -3236,6 +3241,14 @@ static int run_impl(dp_sim* s, long long steps, int kind, float* ms) {
             CK(cudaGetLastError());
         }
         RET(check_device_error(s));
+        // a region without room leaves its brick's lists empty, and unless the steps
+        // stopped there, what the chunk went on to do does not count: not even a
+        // force that became infinite, or the longest row
+        const bool void_chunk = !groups && s->bricks && s->hstat->cell_overflow > s->brick_cap;
+        if (void_chunk) {
+            s->hstat->nonfinite = 0;
+            s->hstat->max_neighbors = 0;
+        }
         if (s->hstat->nonfinite) {
             s->hstat->nonfinite = 0;
             RET(write_status(s));
@@ -3244,17 +3257,26 @@ static int run_impl(dp_sim* s, long long steps, int kind, float* ms) {
         bool grown = false;
         RET(grow_after_overflow(s, &grown));
         if (grown) {
-            if (!backed_up) return fail(DP_ERR_OVERFLOW, "neighbour list overflow without a pending build");
-            if (++retries > 8) return fail(DP_ERR_OVERFLOW, "neighbour list keeps overflowing");
-            RET(restore_state(s));
-            s->hstat->step = step0;
+            const long long before = groups ? s->hstat->step - step0 : 0;  // steps that stand
+            if (!groups && !backed_up) return fail(DP_ERR_OVERFLOW, "neighbour list overflow without a pending build");
+            retries = before > 0 ? 0 : retries + 1;
+            if (retries > 8) return fail(DP_ERR_OVERFLOW, "neighbour list keeps overflowing");
+            if (!groups) {
+                RET(restore_state(s));
+                s->hstat->step = step0;
+            }
             s->hstat->need_rebuild = 1;
             RET(write_status(s));
-            continue;  // replay the chunk with the larger capacity
+            if (groups)
+                s->launches_last += 1 + s->hstat->groups * g->launches +
+                                    (s->hstat->rebuilds - rebuilds0) * g->rebuild_launches;
+            done += before;
+            continue;  // the build again, and the steps from there (or all of the chunk)
         }
         s->launches_last += (groups ? 1 + s->hstat->groups * g->launches : g->launches) +
                             (s->hstat->rebuilds - rebuilds0) * g->rebuild_launches;
         done += c;
+        retries = 0;
     }
     if (ms) {
         CK(cudaEventRecord(s->ev1, s->stream));
