@@ -338,6 +338,15 @@ __device__ __forceinline__ void dp_pair_eval_f64(const dp_pair_args& a, long lon
 }
 #endif
 
+// A load of what the step before wrote. LIVE: this kernel's blocks were placed while
+// that step still ran (dp_step_lists), so the value was not read-only for the whole
+// of the kernel's life and a read-only load may not be used, nor one that the
+// compiler could move across the wait.
+template <bool LIVE, typename T>
+__device__ __forceinline__ T dp_fetch(const T* p) {
+    return LIVE ? *p : __ldg(p);
+}
+
 // Window of the two-pass loop: one thread per particle evaluates 64 listed
 // neighbours at a time (mixture of 256,000, 150 listed: 320 / 298 / 307 us a
 // step with 32 / 64 / 128; 108,000 LJ, 95 listed: 91 / 87 / 84; lists of a
@@ -362,12 +371,12 @@ __device__ __forceinline__ void dp_pair_eval_f64(const dp_pair_args& a, long lon
 // double-loop and vectorised force and energy methods,
 // dompap/potential.py:103-160,191-250,298-324); lane `lane` takes slots
 // lane, lane + LANES, ...  listed: the row's length if the caller knows it.
-template <int ACC, int LANES = 1, bool ALL = false>
+template <int ACC, int LANES = 1, bool ALL = false, bool LIVE = false>
 __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long long i, double* f, int lane = 0,
                                                   int listed = -1) {
     constexpr int D = DP_DIM;
     const long long n = a.n;
-    const shadow_t* __restrict__ sh = (const shadow_t*)a.shadow;
+    const shadow_t* sh = (const shadow_t*)a.shadow;
     uint32_t ui[D];
     int ti = 0;
 #if DP_PMODE == 1
@@ -376,7 +385,7 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
     dp_pair_acc A;
 #if DP_FF
     typedef typename dp_fixed64_t<D>::type fx_t;
-    const fx_t* __restrict__ p64 = (const fx_t*)a.pos64;
+    const fx_t* p64 = (const fx_t*)a.pos64;
     const bool ff_ok = a.status->far == 0;  // single-shift image == nearest image
     unsigned long long Xi[D];
     if (ff_ok) {
@@ -417,7 +426,7 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
                 // over n < m with sigma(n, m), epsilon(n, m)
                 if ((ACC == DP_ACC_VIRIAL || ACC == DP_ACC_ENERGY_UPPER) && dp_upper_skip(a, i, j)) continue;
                 uint32_t uj[D];
-                dp_shadow_unpack<D>(__ldg(sh + j), uj);
+                dp_shadow_unpack<D>(dp_fetch<LIVE>(sh + j), uj);
                 float df[D];
                 if (dp_shadow_q<D>(ui, uj, a.unit, df) <= a.cut2f) kept[q] |= 1u << t;
             }
@@ -446,7 +455,7 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
 #endif
 #if DP_REAL_IS_FLOAT
             uint32_t uj[D];
-            dp_shadow_unpack<D>(__ldg(sh + j), uj);
+            dp_shadow_unpack<D>(dp_fetch<LIVE>(sh + j), uj);
             float df[D];
             const float qf = dp_shadow_q<D>(ui, uj, a.unit, df);
             dp_pair_eval<ACC>(a, i, j, ti, tj, qf, df, A);
@@ -572,7 +581,7 @@ __device__ __forceinline__ int dp_build_row(const dp_pair_args& a, const dp_list
                                             bool far) {
     constexpr int D = DP_DIM;
     const long long n = a.n;
-    const shadow_t* __restrict__ sh = (const shadow_t*)a.shadow;
+    const shadow_t* sh = (const shadow_t*)a.shadow;
     const shadow_t shi = sh[i];
     uint32_t ui[D];
     dp_shadow_unpack<D>(shi, ui);
@@ -584,7 +593,7 @@ __device__ __forceinline__ int dp_build_row(const dp_pair_args& a, const dp_list
         bool in = false;
         if (j < (int)n && j != (int)i) {
             uint32_t uj[D];
-            dp_shadow_unpack<D>(__ldg(sh + j), uj);
+            dp_shadow_unpack<D>(dp_fetch<true>(sh + j), uj);
             float df[D];
             const float q = dp_shadow_q<D>(ui, uj, a.unit, df);
             in = q <= l.hi2;
@@ -617,7 +626,7 @@ __device__ __forceinline__ int dp_build_row(const dp_pair_args& a, const dp_list
 // lane integrates. Below a few tens of thousands of particles this spreads the
 // pair loops over LANES times more threads than dp_step, whose one thread per
 // particle leaves most SMs idle.
-template <int LANES, bool ALL = false>
+template <int LANES, bool ALL = false, bool LIVE = false>
 __device__ __forceinline__ void dp_step_split(const dp_pair_args& a, const dp_int_args& b, const dp_list_args* own) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long i = t / LANES;
@@ -632,7 +641,7 @@ __device__ __forceinline__ void dp_step_split(const dp_pair_args& a, const dp_in
         ref_far = a.status->far != 0;
         if (active) listed = dp_build_row(a, *own, i, lane, ref_far != 0);
     }
-    if (active) dp_particle_sum<DP_ACC_FORCE, LANES, ALL>(a, i, f, lane, listed);
+    if (active) dp_particle_sum<DP_ACC_FORCE, LANES, ALL, LIVE>(a, i, f, lane, listed);
     // every lane of the warp takes part in the shuffles (groups past the
     // last particle add zeros)
 #pragma unroll
@@ -674,7 +683,7 @@ extern "C" __global__ void DP_STEP_BOUNDS dp_step_quad(dp_pair_args a, dp_int_ar
 extern "C" __global__ void __launch_bounds__(256, DP_LISTS_BLOCKS) dp_step_lists(dp_pair_args a, dp_int_args b, dp_list_args l) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    dp_step_split<32>(a, b, &l);
+    dp_step_split<32, false, true>(a, b, &l);
 }
 
 // ---------------------------------------------------------------------------
