@@ -156,7 +156,7 @@ __device__ __forceinline__ void dp_batch_steps(const dp_batch_args& a) {
         // the noise terms in float32, as the single-system integrator
         const float c2f = (float)c[2], c3f = (float)c[3];
         // list of this replica: chunk c of particle p at [(c n + p) 8]
-        uint16_t* __restrict__ nl = a.nlist ? a.nlist + off * (long long)a.kmax : nullptr;
+        uint16_t* nl = a.nlist ? a.nlist + off * (long long)a.kmax : nullptr;
         bool use_list = nl != nullptr;  // cleared for the rest of the launch if the list overflows
 
         const long long step0 = a.st->step;  // advanced by the host-side graph after this launch
@@ -319,17 +319,17 @@ __device__ __forceinline__ void dp_batch_steps(const dp_batch_args& a) {
                     p = slot;
                     const int cnt = a.ncnt[off + p];
                     // one 16-byte load per 8 entries, two chunks ahead of the
-                    // pairs being evaluated
-                    const uint4* __restrict__ rowc = (const uint4*)nl + p;
+                    // pairs being evaluated (not a read-only load: this launch writes the lists)
+                    const uint4* rowc = (const uint4*)nl + p;
                     const int nch = (cnt + 7) >> 3;
                     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
                     auto walk = [&](bool sampled) {
-                        uint4 c1 = nch > 0 ? __ldg(rowc) : zero;
-                        uint4 c2 = nch > 1 ? __ldg(rowc + n) : zero;
+                        uint4 c1 = nch > 0 ? *rowc : zero;
+                        uint4 c2 = nch > 1 ? rowc[n] : zero;
                         for (int ch = 0; ch < nch; ++ch) {
                             const uint4 cur = c1;
                             c1 = c2;
-                            c2 = ch + 2 < nch ? __ldg(rowc + (long long)(ch + 2) * n) : zero;
+                            c2 = ch + 2 < nch ? rowc[(long long)(ch + 2) * n] : zero;
                             const int m = cnt - 8 * ch;
                             const uint32_t w[4] = {cur.x, cur.y, cur.z, cur.w};
 #pragma unroll

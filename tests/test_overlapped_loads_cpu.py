@@ -1,7 +1,8 @@
 """Kernels whose blocks are placed while the launch before still runs
 (griddepcontrol.wait): what that launch writes is not read-only for the whole of
 such a kernel's life, so it may not be read through the read-only path (__ldg,
-const __restrict__). Checked on the source of everything such a kernel calls."""
+const __restrict__). Neither may a kernel so read what it writes itself. Checked
+on the source of everything such a kernel calls."""
 import os
 import re
 
@@ -68,3 +69,9 @@ def test_no_read_only_loads_of_live_data(files, kernels):
         assert "dp_particle_sum<DP_ACC_FORCE, LANES, ALL, LIVE>" in split
         assert "dp_fetch<LIVE>(sh" in "\n".join(functions["dp_particle_sum"])
         assert "dp_fetch<true>(sh" in "\n".join(functions["dp_build_row"])
+
+
+def test_replica_lists_are_read_with_plain_loads():
+    """dp_batch_steps builds its lists and walks them in one launch."""
+    body = "\n".join(_functions(_source("batch_kernels.cuh"))["dp_batch_steps"])
+    assert "__ldg" not in body and "__restrict__" not in body
