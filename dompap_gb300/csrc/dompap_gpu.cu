@@ -109,6 +109,7 @@ struct ShadowArgs {
     dp_dev_status* st;
     long long n;
     double scale64[DP_MAX_DIM];
+    int shift64[DP_MAX_DIM];
     double box[DP_MAX_DIM];
 };
 
@@ -142,6 +143,7 @@ __global__ void k_shadow(ShadowArgs a) {
         }
         X[k] = dp_fixed64_of(p);
         u[k] = (uint32_t)(X[k] >> 32);
+        X[k] <<= a.shift64[k];
     }
     ((typename dp_shadow_t<D>::type*)a.shadow)[i] = dp_shadow_pack<D>(u);
     ((typename dp_fixed64_t<D>::type*)a.pos64)[i] = dp_fixed64_pack<D>(X);
@@ -1320,6 +1322,7 @@ __global__ void k_wrap(dp_int_args a) {
         if (im != im0) a.img[o] = im;
         X[k] = fixed64_wrapped(x, a.box[k], a.scale64[k]);
         u[k] = (uint32_t)(X[k] >> 32);
+        X[k] <<= a.shift64[k];
     }
     ((typename dp_shadow_t<D>::type*)a.shadow_out)[i] = dp_shadow_pack<D>(u);
     ((typename dp_fixed64_t<D>::type*)a.pos64_out)[i] = dp_fixed64_pack<D>(X);
@@ -1865,6 +1868,7 @@ struct dp_sim {
     void* shadow = nullptr;
     void* shadow_ref = nullptr;
     void* pos64 = nullptr;
+    int shift64[DP_MAX_DIM] = {0, 0, 0, 0};  // the 64-bit fixed point is kept modulo L / 2^shift64 (update_shift64)
     size_t shadow_bytes = 0;
     double *bk_pos = nullptr, *bk_vel = nullptr, *bk_beta = nullptr;
     int32_t* bk_img = nullptr;
@@ -2023,6 +2027,7 @@ static int launch_shadow(dp_sim* s) {
     a.st = s->dstat;
     a.n = s->n;
     for (int k = 0; k < DP_MAX_DIM; ++k) a.scale64[k] = 18446744073709551616.0 / ((k < s->dim) ? s->box[k] : 1.0);
+    memcpy(a.shift64, s->shift64, sizeof(a.shift64));
     for (int k = 0; k < DP_MAX_DIM; ++k) a.box[k] = (k < s->dim) ? s->box[k] : 1.0;
     CK(cudaMemsetAsync(&s->dstat->far, 0, sizeof(int32_t), s->stream));
     const unsigned g = grid_for(s->n, kBlock);
@@ -2178,6 +2183,36 @@ static int configure_bricks(dp_sim* s) {
     return DP_OK;
 }
 
+// Pre-filter threshold: a pair is skipped only when its float32 distance,
+// whose error is < 1e-6 relative plus a few L / 2^32, certainly exceeds
+// r_cut * sigma_max.
+static float prefilter_cut2(const dp_sim* s) {
+    double lmax = 0.0;
+    for (int k = 0; k < s->dim; ++k) lmax = std::max(lmax, s->box[k]);
+    const double reach = s->r_cut * s->sig_max;
+    if (!std::isfinite(reach)) return INFINITY;
+    const double rr = reach * (1.0 + 1e-5) + 8.0 * lmax / 4294967296.0 * std::sqrt((double)s->dim) + 1e-30;
+    return (float)(rr * rr * (1.0 + 1e-6));
+}
+
+// A pair that passes the pre-filter is closer than `most` on every axis, so its
+// displacement is known from the positions modulo L / 2^shift64 > 4 most, and
+// their 64 bits hold that many more behind the point of the double-float
+// arithmetic (dpff_from_fixed; shifting the differences instead cost the
+// 256,000-particle mixture 2.5 %).
+static int update_shift64(dp_sim* s) {
+    const double cut = std::sqrt((double)prefilter_cut2(s));
+    int shift[DP_MAX_DIM] = {0, 0, 0, 0};
+    for (int k = 0; k < s->dim; ++k) {
+        const double most = 1.001 * cut + 16.0 * s->box[k] / 4294967296.0;
+        while (shift[k] < 16 && most * (double)(8LL << shift[k]) < s->box[k]) ++shift[k];
+    }
+    if (memcmp(shift, s->shift64, sizeof(shift)) == 0) return DP_OK;
+    memcpy(s->shift64, shift, sizeof(shift));
+    s->version++;
+    return launch_shadow(s);
+}
+
 static int configure_nl(dp_sim* s) {
     if (!s->nl_config_dirty) return DP_OK;
     if (!s->have_box) return fail(DP_ERR_ARG, "box not set");
@@ -2234,6 +2269,7 @@ static int configure_nl(dp_sim* s) {
             RET(dalloc_t(&s->bk_order, n));
         }
     }
+    RET(update_shift64(s));
     s->bricks_off = false;
     RET(configure_bricks(s));
     RET(ensure_list(s));
@@ -2473,7 +2509,7 @@ static void fill_pair_args(const dp_sim* s, dp_pair_args& a, double* out) {
     for (int k = 0; k < DP_MAX_DIM; ++k) a.box[k] = (k < s->dim) ? s->box[k] : 1.0;
     fill_scale(s, nullptr, a.unit);
     for (int k = 0; k < DP_MAX_DIM; ++k) {
-        const double u64 = ((k < s->dim) ? s->box[k] : 1.0) / 18446744073709551616.0;
+        const double u64 = ((k < s->dim) ? s->box[k] : 1.0) / 18446744073709551616.0 / (double)(1LL << s->shift64[k]);
         a.unit64_hi[k] = (float)u64;
         a.unit64_lo[k] = (float)(u64 - (double)(float)u64);
     }
@@ -2498,18 +2534,7 @@ static void fill_pair_args(const dp_sim* s, dp_pair_args& a, double* out) {
         a.f32_const[2] = f.z;
         a.f32_const[3] = f.w;
     }
-    // Pre-filter threshold: a pair is skipped only when its float32 distance,
-    // whose error is < 1e-6 relative plus a few L / 2^32, certainly exceeds
-    // r_cut * sigma_max.
-    double lmax = 0.0;
-    for (int k = 0; k < s->dim; ++k) lmax = std::max(lmax, s->box[k]);
-    const double reach = s->r_cut * s->sig_max;
-    if (std::isfinite(reach)) {
-        const double rr = reach * (1.0 + 1e-5) + 8.0 * lmax / 4294967296.0 * std::sqrt((double)s->dim) + 1e-30;
-        a.cut2f = (float)(rr * rr * (1.0 + 1e-6));
-    } else {
-        a.cut2f = INFINITY;
-    }
+    a.cut2f = prefilter_cut2(s);
 }
 
 static bool use_mlp_tcgen05(const dp_sim* s) {
@@ -2635,6 +2660,7 @@ static void fill_int_args(const dp_sim* s, dp_int_args& a, long long step_offset
     for (int k = 0; k < DP_MAX_DIM; ++k) a.box[k] = (k < s->dim) ? s->box[k] : 1.0;
     fill_scale(s, nullptr, a.unit);
     for (int k = 0; k < DP_MAX_DIM; ++k) a.scale64[k] = 18446744073709551616.0 / ((k < s->dim) ? s->box[k] : 1.0);
+    memcpy(a.shift64, s->shift64, sizeof(a.shift64));
     a.thr = (0.5 * s->skin) * (0.5 * s->skin);
     bracket(s, 0.5 * s->skin, &a.thr_lo, &a.thr_hi);
     a.dt = s->dt;

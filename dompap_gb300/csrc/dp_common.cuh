@@ -50,7 +50,7 @@ struct dp_pair_args {
     const double* isig_tab;  // 1 / sigma per type pair (DP_PMODE == 1)
     const float2* ff_tab;    // DP_PMODE == 1: per type pair DP_FF_PARAMS double-floats (see ff_const)
     const float4* f32_tab;   // DP_PMODE == 1: per type pair sigma, 1/sigma, epsilon
-    const void* pos64;       // 64-bit fixed-point positions (X = x 2^64 / L), one vector per particle
+    const void* pos64;       // 64-bit fixed-point positions (X = x 2^(64 + shift64) / L mod 2^64), one vector per particle
     const int32_t* order;    // particle id held by each slot (slots are in cell order after a rebuild)
     double* out;
     double* partial;
@@ -60,7 +60,7 @@ struct dp_pair_args {
     int upper;               // DP_PMODE == 2: parameters of (min, max) of the two ids (Newton's-third-law loop)
     double box[DP_MAX_DIM];
     float unit[DP_MAX_DIM];  // L / 2^32 per axis
-    float unit64_hi[DP_MAX_DIM];  // L / 2^64 per axis as a double-float
+    float unit64_hi[DP_MAX_DIM];  // L / 2^(64 + shift64) per axis as a double-float
     float unit64_lo[DP_MAX_DIM];
     double sigma;            // DP_PMODE == 0
     double inv_sigma;        // DP_PMODE == 0

@@ -110,11 +110,13 @@ __device__ __forceinline__ dpff dpff_rcp(dpff q) {
     return dpff_quick_two_sum(y, y * fmaf(e, e, e));
 }
 
-// The 64-bit fixed-point displacement v (units 2^-64 L) times L, U = L / 2^32 as
+// The 64-bit fixed-point displacement v (units 2^-64 M) times M, U = M / 2^32 as
 // a double-float, u24 = U.hi / 2^24. v = h 2^32 + l: what the nearest float of h
 // leaves of it (at most 64) and the upper 24 bits of l make one 31-bit integer
 // (a funnel shift), so three conversions carry ~48 leading bits of v; what is
-// dropped lies below 2^-56 L. An h that rounds up to 2^31 saturates on the way
+// dropped lies below 2^-56 M, so M is not the box but at most eight times the
+// cutoff (dp_sim::shift64): with M = 10,000 the force error was 30 times that of a
+// short box. An h that rounds up to 2^31 saturates on the way
 // back, one short of it. (An int64 split into 22 / 22 / 20 bits took the same
 // three conversions and twice the instructions; rounding h towards zero, or
 // leaving the product unnormalised, saves a few but costs a bit of accuracy.)

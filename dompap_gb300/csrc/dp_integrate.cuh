@@ -31,6 +31,7 @@ struct dp_int_args {
     long long n;
     double box[DP_MAX_DIM];
     double scale64[DP_MAX_DIM];  // 2^64 / L
+    int shift64[DP_MAX_DIM];     // left shift of the 64-bit fixed point that is stored
     float unit[DP_MAX_DIM];      // L / 2^32
     double thr;                  // (skin/2)^2
     float thr_lo, thr_hi;        // float32 bracket of thr for the shadow test
@@ -196,6 +197,7 @@ __device__ __forceinline__ bool dp_integrate_one(const dp_int_args& a, long long
         }
         X[k] = dp_fixed64_of(p);
         u[k] = (uint32_t)(X[k] >> 32);
+        if (WRITE64) X[k] <<= a.shift64[k];
         a.vel[o] = v;
         a.pos_out[o] = x;
         xs[k] = x;

@@ -388,17 +388,9 @@ __device__ __forceinline__ double dp_particle_sum(const dp_pair_args& a, long lo
     const fx_t* p64 = (const fx_t*)a.pos64;
     const bool ff_ok = a.status->far == 0;  // single-shift image == nearest image
     unsigned long long Xi[D];
-    if (ff_ok) {
-        // the pre-filter runs on the upper words of the 64-bit fixed point
-        dp_fixed64_unpack<D>(p64[i], Xi);
-#pragma unroll
-        for (int k = 0; k < D; ++k) ui[k] = (uint32_t)(Xi[k] >> 32);
-    } else {
-        dp_shadow_unpack<D>(sh[i], ui);
-    }
-#else
-    dp_shadow_unpack<D>(sh[i], ui);
+    if (ff_ok) dp_fixed64_unpack<D>(p64[i], Xi);
 #endif
+    dp_shadow_unpack<D>(sh[i], ui);
     // Two passes over windows of up to DP_WINDOW listed neighbours. Pass 1 runs
     // the float32 pre-filter on the shadows and keeps a bit per neighbour that
     // may lie within r_cut * sigma_max; pass 2 evaluates the pair terms of
