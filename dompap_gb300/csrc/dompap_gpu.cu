@@ -26,6 +26,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <cctype>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -1599,7 +1600,7 @@ struct PairLib {
     cudaKernel_t split[2][4] = {{nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}};
     // no neighbour list (dompap's double-loop methods): fused step, forces, energy
     cudaKernel_t step_all = nullptr, forces_all = nullptr, energy_all = nullptr;
-    // bricks of cells (not in 4-D, with dense parameters or in the surrogate
+    // bricks of cells (not in 4-D, with dense parameters, costly potentials or in the surrogate
     // program): fused step with 1 or 4 lanes per particle, forces, scalars
     cudaKernel_t step_brick[2] = {nullptr, nullptr};
     cudaKernel_t forces_brick = nullptr, energy_brick = nullptr, virial_brick = nullptr, laplacian_brick = nullptr;
@@ -3639,9 +3640,59 @@ static std::string hexd(double v) {
     return buf;
 }
 
-// The program has the brick kernels.
-static bool brick_program(int dim, int precision, int pmode) {
-    return dim <= 3 && precision == DP_PREC_FP32 && pmode != DP_PAIR_DENSE;
+// What a warp pays for the force of a generated potential, by the calls and
+// divisions in dp_pair_f: 1 for those of a few instructions (exp, log, sqrt, a
+// division), 2 for the hyperbolic ones and cbrt, 4 for those with long or
+// branching code (sin, cos, pow, erf and anything else).
+static int pair_cost(const std::string& src) {
+    size_t at = src.find("dp_pair_f(");
+    at = at == std::string::npos ? at : src.find('{', at);
+    if (at == std::string::npos) return 0;
+    static const char* const free_of_charge[] = {"R", "dp_k", "dp_ipow", "fabs", "fmin", "fmax", "floor", "ceil", "const",
+                                                 "return", "if"};
+    static const char* const cheap[] = {"exp", "exp2", "expm1", "log", "log2", "log1p", "sqrt", "rsqrt"};
+    static const char* const fair[] = {"tanh", "sinh", "cosh", "cbrt"};
+    auto in = [](const std::string& name, const char* const* list, size_t m) {
+        for (size_t k = 0; k < m; ++k)
+            if (name == list[k]) return true;
+        return false;
+    };
+    int cost = 0, depth = 0;
+    for (; at < src.size(); ++at) {
+        const char ch = src[at];
+        if (ch == '{') ++depth;
+        if (ch == '}' && --depth == 0) break;
+        if (ch == '/') cost += 1;
+        if (!std::isalpha((unsigned char)ch) && ch != '_') {
+            // a number: none of its letters is a name
+            if (std::isdigit((unsigned char)ch))
+                while (at + 1 < src.size() && (std::isalnum((unsigned char)src[at + 1]) || src[at + 1] == '.')) ++at;
+            continue;
+        }
+        size_t end = at;
+        while (end < src.size() && (std::isalnum((unsigned char)src[end]) || src[end] == '_')) ++end;
+        const std::string name = src.substr(at, end - at);
+        at = end - 1;
+        if (end >= src.size() || src[end] != '(') continue;  // (the templates' names end in '>')
+        if (in(name, free_of_charge, sizeof(free_of_charge) / sizeof(char*))) continue;
+        cost += in(name, cheap, sizeof(cheap) / sizeof(char*)) ? 1 : (in(name, fair, sizeof(fair) / sizeof(char*)) ? 2 : 4);
+    }
+    return cost;
+}
+
+// The program has the brick kernels: not for costly potentials. The one pass of
+// the brick loop evaluates the force for every listed entry of a warp with a pair
+// inside the cut (two in three listed ones, in eight copies of its code); the two passes over
+// lists of slots only for kept ones, in one copy. us a step, 108,000 / 1,048,576
+// particles, bricks against slots: LJ 73 / 373 against 91 / 591, three exp (3) 91 /
+// 566 against 99 / 654, pow (4) 119 / 629 against 109 / 714, two pow (8) 145 against
+// 121, LJ + exp (cos + sin) (9) 131 / 852 against 119 / 777, the costly test potential
+// with eight more such terms 956 / 6,053 against 318 / 2,476. (Two passes on the bricks
+// lost to slots everywhere: 459 / 2,692 on the last, 98 / 619 on LJ.)
+constexpr int kBrickCost = 6;
+
+static bool brick_program(int dim, int precision, int pmode, const std::string& pot_src) {
+    return dim <= 3 && precision == DP_PREC_FP32 && pmode != DP_PAIR_DENSE && pair_cost(pot_src) < kBrickCost;
 }
 
 static std::string pair_program(int dim, int precision, int pmode, bool sig_one, bool eps_one,
@@ -3674,7 +3725,7 @@ static std::string pair_program(int dim, int precision, int pmode, bool sig_one,
     src += pot_src;
     src += "\n// ---- pair kernels ----\n";
     src += dp_src_pair;
-    if (brick_program(dim, precision, pmode) && !with_batch) {
+    if (brick_program(dim, precision, pmode, pot_src) && !with_batch) {
         src += "\n#define DP_BRICKS 1\n#define DP_BRICK_BLOCKS " + std::to_string(brick_blocks) + "\n";
         src += dp_src_brick;
     }
