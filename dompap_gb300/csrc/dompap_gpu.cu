@@ -3689,10 +3689,23 @@ static int pair_cost(const std::string& src) {
 // 121, LJ + exp (cos + sin) (9) 131 / 852 against 119 / 777, the costly test potential
 // with eight more such terms 956 / 6,053 against 318 / 2,476. (Two passes on the bricks
 // lost to slots everywhere: 459 / 2,692 on the last, 98 / 619 on LJ.)
-constexpr int kBrickCost = 6;
+constexpr int kCostlyPair = 6;
 
 static bool brick_program(int dim, int precision, int pmode, const std::string& pot_src) {
-    return dim <= 3 && precision == DP_PREC_FP32 && pmode != DP_PAIR_DENSE && pair_cost(pot_src) < kBrickCost;
+    return dim <= 3 && precision == DP_PREC_FP32 && pmode != DP_PAIR_DENSE && pair_cost(pot_src) < kCostlyPair;
+}
+
+// The generated functions of a costly potential as calls: in float32 their code,
+// once in every kernel that evaluates pairs and eight times in an unrolled loop, outgrows the
+// registers of the loop around it and the instruction caches. us a step, inlined
+// and called, costly test potential with 0 / 1 / 8 / 16 more terms, 1,048,576
+// particles: 656 / 851 / 2,294 / 4,746 and 620 / 795 / 1,980 / 4,271; 512
+// replicas of 2,048, 0 / 4 / 8 more: 1,981 / 4,351 / 17,390 and 841 / 1,959 / 3,311.
+// (Cheap ones stay inline: 512 replicas of a Gaussian on LJ 489 against 500.)
+static std::string called_pair_functions(std::string src) {
+    const std::string was = "__forceinline__ R dp_pair_", now = "__noinline__ R dp_pair_";
+    for (size_t at = 0; (at = src.find(was, at)) != std::string::npos; at += now.size()) src.replace(at, was.size(), now);
+    return src;
 }
 
 static std::string pair_program(int dim, int precision, int pmode, bool sig_one, bool eps_one,
@@ -3722,7 +3735,7 @@ static std::string pair_program(int dim, int precision, int pmode, bool sig_one,
     if (precision == DP_PREC_MLP) src += dp_src_umma;
     if (precision == DP_PREC_FP64) src += dp_src_ff;
     src += "\n// ---- generated pair potential ----\n";
-    src += pot_src;
+    src += precision == DP_PREC_FP32 && pair_cost(pot_src) >= kCostlyPair ? called_pair_functions(pot_src) : pot_src;
     src += "\n// ---- pair kernels ----\n";
     src += dp_src_pair;
     if (brick_program(dim, precision, pmode, pot_src) && !with_batch) {
@@ -3743,9 +3756,12 @@ static std::string pair_program(int dim, int precision, int pmode, bool sig_one,
 // harmonic: 3 % faster) and for per-type or per-pair tables (~600 bytes of
 // spills under 40 registers; the Wahnstrom mixture ran 17 % slower with 6);
 // 6 (40 registers) for the float32 pair loop and in 2 dimensions, where the
-// occupancy is worth more (7-8 % faster than with 4).
-static int step_blocks_for(int dim, int precision, int pmode) {
-    if (pmode != DP_PAIR_CONST) return 4;
+// occupancy is worth more (7-8 % faster than with 4), up to costs where it is the
+// pair terms' registers that count (the costly test potential with 1 / 8 more terms:
+// 6 CTAs 795 / 2,099, 4 CTAs 858 / 1,980).
+constexpr int kStepCost = 40;
+static int step_blocks_for(int dim, int precision, int pmode, int cost) {
+    if (pmode != DP_PAIR_CONST || (precision == DP_PREC_FP32 && cost >= kStepCost)) return 4;
     return precision == DP_PREC_FP64 && dim >= 3 ? 4 : 6;
 }
 
@@ -3762,7 +3778,8 @@ static int lists_blocks_for(long long n) { return n < 3072 ? 2 : 4; }
 static int rebuild_pair_lib(dp_sim* s) {
     const bool sig_one = s->pmode == DP_PAIR_CONST && s->sigma == 1.0;
     const bool eps_one = s->pmode == DP_PAIR_CONST && s->epsilon == 1.0;
-    const int step_blocks = s->step_blocks ? s->step_blocks : step_blocks_for(s->dim, s->precision, s->pmode);
+    const int step_blocks =
+        s->step_blocks ? s->step_blocks : step_blocks_for(s->dim, s->precision, s->pmode, pair_cost(s->pot_src));
     const std::string src =
         pair_program(s->dim, s->precision, s->pmode, sig_one, eps_one, s->pot_src, false, step_blocks,
                      s->step_blocks ? s->step_blocks : brick_blocks_for(s->n),
@@ -3812,7 +3829,7 @@ int dp_get_step_launch(dp_sim* s, int* lanes, int* blocks_per_sm) {
                            : step_lanes(s);
     *blocks_per_sm = s->step_blocks ? s->step_blocks
                      : brick        ? brick_blocks_for(s->n)
-                                    : step_blocks_for(s->dim, s->precision, s->pmode);
+                                    : step_blocks_for(s->dim, s->precision, s->pmode, pair_cost(s->pot_src));
     return DP_OK;
 }
 
@@ -4828,7 +4845,7 @@ static int nvrtc_check_impl(int dim, int precision, int pair_mode, int with_batc
     if (pair_mode < DP_PAIR_CONST || pair_mode > DP_PAIR_DENSE) return fail(DP_ERR_ARG, "unknown pair mode");
     const bool one = pair_mode == DP_PAIR_CONST;
     const std::string src = pair_program(dim, precision, pair_mode, one, one, device_source, with_batch != 0,
-                                         step_blocks_for(dim, precision, pair_mode));
+                                         step_blocks_for(dim, precision, pair_mode, pair_cost(device_source)));
     std::vector<char> cubin;
     RET(nvrtc_cubin(src, &cubin, resource_log, true, true));
     if (cubin_bytes) *cubin_bytes = (int64_t)cubin.size();

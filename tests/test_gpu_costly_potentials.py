@@ -40,8 +40,9 @@ def test_which_lists(potential):
     if potential == "Harmonic repulsive":  # its cut is 1: too few neighbours for bricks
         sim.set_neighbor_list(skin=2.0, max_number_of_neighbors=256, method_str="cell list")
     sim.update_neighbor_list(check=False)
-    # 4 lanes a particle either way; bricks are compiled for 4 CTAs an SM, slots for 6
-    assert sim.get_step_launch() == ((4, 4) if potential in CHEAP else (4, 6))
+    # 4 lanes a particle either way; bricks are compiled for 4 CTAs an SM, slots for
+    # 6, or 4 where the pair terms need the registers
+    assert sim.get_step_launch() == ((4, 6) if potential in DEAR[1:] else (4, 4))
 
 
 def test_costly_step_time():
@@ -57,8 +58,30 @@ def test_costly_step_time():
     assert ms["costly"] <= 7.0 * ms["lj"]
 
 
-def test_forces_agree_with_float64():
-    a = _sim(COSTLY, (14, 14, 14))
+def test_costly_replicas_time():
+    """256 replicas of 2,048: the costly force a dozen times Lennard-Jones' at most
+    (8 here; more than 30 where it was inlined into every entry of the loop)."""
+    from dompap_gb300.batched import Replicas, ReplicaSpec
+    from dompap_gb300.positions import FCC, generate_positions
+
+    scale = (4 / 0.8) ** (1 / 3)
+    pos, box = generate_positions(FCC, (8, 8, 8), (1.0,) * 3) * scale, np.full(3, 8 * scale)
+    rng = np.random.default_rng(3)
+    specs = []
+    for _ in range(256):
+        p = pos + rng.normal(0.0, 0.05, size=pos.shape)
+        specs.append(ReplicaSpec(p - np.floor(p / box) * box, rng.normal(size=p.shape), box, 1.0))
+    ms = {}
+    for name, potential in (("lj", LJ), ("costly", COSTLY)):
+        replicas = Replicas(specs, potential, 3.0, seed=1)
+        replicas.run(3)
+        ms[name] = min(replicas.run(20) for _ in range(3))
+    assert ms["costly"] <= 12.0 * ms["lj"]
+
+
+@pytest.mark.parametrize("cells", [(5, 5, 5), (14, 14, 14)])
+def test_forces_agree_with_float64(cells):
+    a = _sim(COSTLY, cells)
     f = a.get_forces()
     u, w = a.get_potential_energy(), a.get_virial()
     a.set_precision("fp64")
