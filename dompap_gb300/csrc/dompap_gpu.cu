@@ -385,10 +385,11 @@ __global__ void k_bin_scatter(BinArgs a) {
 
 // Each cell's range ordered by particle id (the atomic ranks are not
 // deterministic; the result is): four lanes a cell, each entry's place the
-// number of smaller ids in its cell (ids and slots of up to kSortCell entries in
-// shared memory; a longer cell by insertion). One thread inserting 25 entries
-// in global memory, each step waiting for the last, took 46 us at 21,000
-// particles (LJ cells), longer than the rest of the binning together.
+// number of smaller ids in its cell. Ids and slots of up to kSortCell entries lie
+// in shared memory, those of a longer cell in `key` and `rank`, which have done
+// their work by now. (Insertion waits for every step before the next: with one
+// thread a cell of 25 entries 46 us at 21,000 particles, longer than the rest of
+// the binning together; cells of 109, in 4-D, 1.5 to 2.2 ms at 262,144.)
 constexpr int kSortLanes = 4;
 constexpr int kSortCell = 48;
 
@@ -399,34 +400,36 @@ __global__ void __launch_bounds__(kBlock) k_bin_sort(BinArgs a) {
     const long long b = (long long)blockIdx.x * (kBlock / kSortLanes) + q;
     const bool cell = b < a.nbins;
     const int lo = cell ? a.bin_start[b] : 0, m = cell ? a.bin_start[b + 1] - lo : 0;
-    const bool ranked = m <= kSortCell;
-    if (ranked) {
-        for (int t = l; t < m; t += kSortLanes) {
-            const int32_t v = a.src_of[lo + t];
+    const bool fits = m <= kSortCell;
+    for (int t = l; t < m; t += kSortLanes) {
+        const int32_t v = a.src_of[lo + t];
+        if (fits) {
             slot[q][t] = v;
             id[q][t] = a.order[v];
+        } else {
+            a.key[lo + t] = a.order[v];
         }
     }
     __syncwarp();
-    if (ranked) {
+    if (fits) {
         for (int t = l; t < m; t += kSortLanes) {
             const int32_t mine = id[q][t];
             int place = 0;
             for (int u = 0; u < m; ++u) place += id[q][u] < mine;
             a.src_of[lo + place] = slot[q][t];
         }
-    } else if (l == 0) {
-        for (int t = lo + 1; t < lo + m; ++t) {
-            const int32_t v = a.src_of[t];
-            const int32_t w = a.order[v];
-            int u = t - 1;
-            while (u >= lo && a.order[a.src_of[u]] > w) {
-                a.src_of[u + 1] = a.src_of[u];
-                --u;
-            }
-            a.src_of[u + 1] = v;
+    } else {
+        for (int t = l; t < m; t += kSortLanes) {
+            const int32_t mine = a.key[lo + t];
+            int place = 0;
+#pragma unroll 4
+            for (int u = 0; u < m; ++u) place += a.key[lo + u] < mine;
+            a.rank[lo + place] = a.src_of[lo + t];
         }
     }
+    __syncwarp();
+    if (!fits)
+        for (int t = l; t < m; t += kSortLanes) a.src_of[lo + t] = a.rank[lo + t];
 }
 
 // --------------------------- permutation of the state ----------------------
@@ -537,7 +540,7 @@ struct NlArgs {
     const int32_t* src_of;     // slot of each entry of the ranges (null: the entries are the slots)
     dp_dev_status* st;
     long long n;
-    long long nl_k, nl_i;      // entry k of slot i at nl[k nl_k + i nl_i]
+    long long nl_k, nl_i;      // k_nl_build_rows: entry k of slot i at nl[k nl_k + i nl_i] (else column-major)
     int kcap;
     int morton;
     int nc[DP_MAX_DIM];
@@ -616,7 +619,7 @@ __global__ void __launch_bounds__(kBlock) k_nl_build_cells(NlArgs a) {
                 inside = sqrt(dp_sqsum_exact<D>(d)) < a.cutoff;
             }
             if (inside) {
-                if (count < a.kcap) a.nl[count * a.nl_k + i * a.nl_i] = j;
+                if (count < a.kcap) a.nl[(long long)count * n + i] = j;
                 ++count;
             }
         }
@@ -947,8 +950,8 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_brick_build(NlArgs a, Bric
                 found[h] += __shfl_sync(0xffffffffu, upto, 3, 4);
                 int left = min(mine, a.kcap - at);
                 if (OUT32) {
-                    int32_t* to = a.nl + at * a.nl_k + i * a.nl_i;
-                    for (; left > 0; --left, to += a.nl_k) {
+                    int32_t* to = a.nl + at * n + i;
+                    for (; left > 0; --left, to += n) {
                         const int s = __clz(m);
                         m &= ~(0x80000000u >> s);
                         *to = rslot[t0 + 32 * c + s];
@@ -1044,7 +1047,7 @@ __global__ void __launch_bounds__(kBlock) k_nl_build_allpairs(NlArgs a) {
                     inside = sqrt(dp_sqsum_exact<D>(d)) < a.cutoff;
                 }
                 if (inside) {
-                    if (count < a.kcap) a.nl[count * a.nl_k + i * a.nl_i] = (int32_t)j;
+                    if (count < a.kcap) a.nl[(long long)count * n + i] = (int32_t)j;
                     ++count;
                 }
             }
