@@ -3202,8 +3202,8 @@ static long long chunk_steps(const dp_sim* s) {
     return c;
 }
 
-// Capture and instantiate, before any step runs, every chunk graph a run of
-// `steps` steps will launch: the chunk lengths, each keyed by the position
+// Capture and instantiate, before any step runs, every graph a run of `steps`
+// steps will launch: the groups, or the chunk lengths, each keyed by the position
 // buffer set that is current when it starts (a fused chunk of odd length
 // leaves the other set current). A timed run then measures launches only.
 static int prepare_one(dp_sim* s, long long c, int kind, bool other_set) {
@@ -3216,17 +3216,29 @@ static int prepare_one(dp_sim* s, long long c, int kind, bool other_set) {
 
 static int prepare_graphs(dp_sim* s, long long steps, int kind) {
     if (steps <= 0) return DP_OK;
+    const long long chunk = chunk_steps(s);
     if (use_groups(s)) {
-        if (prepare_one(s, -1, kind, false) == DP_OK) return DP_OK;
+        // a single step runs without a graph; a chunk may leave either buffer set
+        // current, so that the next can start from either
+        if (steps == 1) return DP_OK;
+        if (prepare_one(s, -1, kind, false) == DP_OK) return steps > chunk ? prepare_one(s, -1, kind, true) : DP_OK;
         // no conditional nodes (conditional_graphs is cleared now): chunks
     }
-    const long long chunk = chunk_steps(s);
     const bool odd = use_fused_step(s) && (chunk & 1);  // each full chunk flips the sets
     const long long full = steps / chunk, rem = steps % chunk;
     if (full >= 1) RET(prepare_one(s, chunk, kind, false));
     if (full >= 2 && odd) RET(prepare_one(s, chunk, kind, true));
     if (rem > 0) RET(prepare_one(s, rem, kind, odd && (full & 1)));
     return DP_OK;
+}
+
+// After steps (hstat is current): what they ran into.
+static int check_run_status(dp_sim* s) {
+    RET(check_device_error(s));
+    if (!s->hstat->nonfinite) return DP_OK;
+    s->hstat->nonfinite = 0;
+    RET(write_status(s));
+    return fail(DP_ERR_NONFINITE, "a force or position became NaN/Inf during run()");
 }
 
 static int run_impl(dp_sim* s, long long steps, int kind, float* ms) {
@@ -3248,6 +3260,19 @@ static int run_impl(dp_sim* s, long long steps, int kind, float* ms) {
         const long long c = std::min(chunk, steps - done);
         const long long step0 = s->hstat->step;  // hstat is current: every path here ends in read_status
         const long long rebuilds0 = s->hstat->rebuilds;
+        // one step on a list that is valid (hstat is current): no rebuild can be due
+        // before it, so it needs no graph
+        if (c == 1 && use_groups(s) && !s->hstat->need_rebuild) {
+            RET(launch_step(s, kind, 0, &s->launches_last, DP_END_CLEAR_FAR));
+            k_advance_step<<<1, 1, 0, s->stream>>>(s->dstat, 1, 1);
+            CK(cudaGetLastError());
+            swap_position_buffers(s);
+            s->launches_last += 1;
+            done += 1;
+            RET(read_status(s));
+            RET(check_run_status(s));
+            continue;
+        }
         GraphEntry* g = nullptr;
         const bool groups = use_groups(s);
         // a chunk needs the backup only if a list build inside it can
@@ -3270,7 +3295,6 @@ static int run_impl(dp_sim* s, long long steps, int kind, float* ms) {
             k_group_start<<<1, 1, 0, s->stream>>>(s->dstat, 0);
             CK(cudaGetLastError());
         }
-        RET(check_device_error(s));
         // a region without room leaves its brick's lists empty, and unless the steps
         // stopped there, what the chunk went on to do does not count: not even a
         // force that became infinite, or the longest row
@@ -3279,11 +3303,7 @@ static int run_impl(dp_sim* s, long long steps, int kind, float* ms) {
             s->hstat->nonfinite = 0;
             s->hstat->max_neighbors = 0;
         }
-        if (s->hstat->nonfinite) {
-            s->hstat->nonfinite = 0;
-            RET(write_status(s));
-            return fail(DP_ERR_NONFINITE, "a force or position became NaN/Inf during run()");
-        }
+        RET(check_run_status(s));
         bool grown = false;
         RET(grow_after_overflow(s, &grown));
         if (grown) {
