@@ -1859,6 +1859,8 @@ struct dp_sim {
     int brick_ext[DP_MAX_DIM] = {1, 1, 1, 1};
     int4 *brick_base = nullptr, *brick_info = nullptr;
     int32_t* brick_slots = nullptr;
+    int bricks_alloc = 0;              // bricks the first two have room for
+    long long brick_slots_alloc = 0;   // entries of brick_slots
     bool brick_pairs = false;  // the float32 pair kernels run on the bricks
     // second set of position buffers: a fused step reads pos/shadow/pos64 and
     // writes these, then the two sets change roles
@@ -2090,7 +2092,13 @@ static int ensure_list(dp_sim* s) {
 constexpr int kBrickMaxCap = 3072;
 
 static int alloc_brick_slots(dp_sim* s, int cap) {
-    RET(dalloc_t(&s->brick_slots, (size_t)s->nbricks * cap));
+    // (grown, never shrunk: a box that is scaled step by step keeps its buffers)
+    const long long need = (long long)s->nbricks * cap;
+    if (need > s->brick_slots_alloc) {
+        s->brick_slots_alloc = 0;
+        RET(dalloc_t(&s->brick_slots, (size_t)need));
+        s->brick_slots_alloc = need;
+    }
     s->brick_cap = cap;
     s->version++;
     return DP_OK;
@@ -2147,9 +2155,13 @@ static int configure_bricks(dp_sim* s) {
                 for (at[3] = 0; at[3] < s->nc[3]; at[3] += 1 << bits[3])
                     base.push_back(make_int4(at[0], at[1], at[2], at[3]));
     s->nbricks = (int)base.size();
-    RET(dalloc_t(&s->brick_base, base.size()));
-    RET(dalloc_t(&s->brick_info, base.size()));
-    CK(cudaMemcpy(s->brick_base, base.data(), base.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    if (s->nbricks > s->bricks_alloc) {
+        s->bricks_alloc = 0;
+        RET(dalloc_t(&s->brick_base, base.size()));
+        RET(dalloc_t(&s->brick_info, base.size()));
+        s->bricks_alloc = s->nbricks;
+    }
+    CK(cudaMemcpyAsync(s->brick_base, base.data(), base.size() * sizeof(int4), cudaMemcpyHostToDevice, s->stream));
     // the box of the brick's cells and everything within the cutoff of it (all of
     // the cells around it at most), with the spread of a random arrangement
     double side[DP_MAX_DIM], volume = 1.0;
