@@ -1979,6 +1979,7 @@ static int dalloc(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
         *p = nullptr;
+        cudaGetLastError();  // not a later launch's
         return fail(DP_ERR_CUDA, std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e));
     }
     return DP_OK;
@@ -1989,10 +1990,19 @@ static int dalloc_t(T** p, size_t count) {
     return dalloc((void**)p, count * sizeof(T));
 }
 
+// A buffer of at least `need` entries; one that could not be had has room for none.
+template <typename T, typename Count>
+static int dgrow_t(T** p, Count need, Count* have) {
+    if (need <= *have) return DP_OK;
+    *have = 0;
+    RET(dalloc_t(p, (size_t)need));
+    *have = need;
+    return DP_OK;
+}
+
 static int ensure_partial(dp_sim* s, long long blocks) {
     if (blocks <= s->partial_alloc) return DP_OK;
-    RET(dalloc_t(&s->partial, (size_t)blocks));
-    s->partial_alloc = blocks;
+    RET(dgrow_t(&s->partial, blocks, &s->partial_alloc));
     s->version++;
     return DP_OK;
 }
@@ -2077,15 +2087,19 @@ static int upload_mass_coefficients(dp_sim* s) {
 }
 
 // --------------------------- neighbour-list configuration -----------------
+// The list's buffers could not be had: nothing may use them before they are.
+static void no_list(dp_sim* s) {
+    s->nl_built = false;
+    s->nl_config_dirty = true;
+}
+
 // Room for kcap entries per particle: 4 bytes each, or 2 in 16-byte chunks
 // (brick lists), whichever is more.
 static int ensure_list(dp_sim* s) {
     const long long need = (long long)std::max(s->kcap, ((s->kcap + 7) & ~7) / 2) * s->n;
-    if (need > s->nl_alloc) {
-        RET(dalloc_t(&s->nl, (size_t)need));
-        s->nl_alloc = need;
-    }
-    return DP_OK;
+    const int rc = dgrow_t(&s->nl, need, &s->nl_alloc);
+    if (rc != DP_OK) no_list(s);
+    return rc;
 }
 
 // Largest region: 117 KB in k_brick_build, 48 KB in the pair kernels.
@@ -2093,11 +2107,10 @@ constexpr int kBrickMaxCap = 3072;
 
 static int alloc_brick_slots(dp_sim* s, int cap) {
     // (grown, never shrunk: a box that is scaled step by step keeps its buffers)
-    const long long need = (long long)s->nbricks * cap;
-    if (need > s->brick_slots_alloc) {
-        s->brick_slots_alloc = 0;
-        RET(dalloc_t(&s->brick_slots, (size_t)need));
-        s->brick_slots_alloc = need;
+    const int rc = dgrow_t(&s->brick_slots, (long long)s->nbricks * cap, &s->brick_slots_alloc);
+    if (rc != DP_OK) {
+        no_list(s);
+        return rc;
     }
     s->brick_cap = cap;
     s->version++;
@@ -2268,12 +2281,13 @@ static int configure_nl(dp_sim* s) {
         s->morton = padded <= (1LL << 26) && pmax <= (1 << bits_per_axis);
         s->nbins = s->morton ? padded : ncell;
         if (s->nbins > s->bins_alloc) {
+            s->bins_alloc = 0;
             RET(dalloc_t(&s->bin_cnt, (size_t)s->nbins));
             RET(dalloc_t(&s->bin_start, (size_t)s->nbins + 1));
             RET(dalloc_t(&s->bin_part, (size_t)((s->nbins + kScanTile - 1) / kScanTile)));
             s->bins_alloc = s->nbins;
         }
-        if (!s->bin_key) {
+        if (!s->bk_order) {  // the last of them
             const size_t n = (size_t)s->n, nd = n * s->dim;
             RET(dalloc_t(&s->bin_key, n));
             RET(dalloc_t(&s->bin_rank, n));
@@ -2299,15 +2313,15 @@ static int configure_nl(dp_sim* s) {
 // classes, masses), allocated once those exist.
 static int ensure_perm_extras(dp_sim* s) {
     const size_t n = (size_t)s->n;
-    if (s->types && !s->sc_types) {
+    if (s->types && !s->bk_types) {
         RET(dalloc_t(&s->sc_types, n));
         RET(dalloc_t(&s->bk_types, n));
     }
-    if (s->mclass && !s->sc_mclass) {
+    if (s->mclass && !s->bk_mclass) {
         RET(dalloc_t(&s->sc_mclass, n));
         RET(dalloc_t(&s->bk_mclass, n));
     }
-    if (s->mass && !s->sc_mass) {
+    if (s->mass && !s->bk_mass) {
         RET(dalloc_t(&s->sc_mass, n));
         RET(dalloc_t(&s->bk_mass, n));
     }
@@ -4278,6 +4292,7 @@ int dp_rdf_counts(dp_sim* s, int type_a, int type_b, const double* edges, int nb
     // edges, the selections' lengths and counts in one buffer of the handle,
     // grown as needed: the last two are cleared together
     if (nbins > s->rdf_bins) {
+        s->rdf_bins = 0;
         RET(dalloc(&s->rdf_buf, (size_t)(nbins + 1) * sizeof(double) + (size_t)(nbins + 1) * sizeof(unsigned long long)));
         s->rdf_bins = nbins;
     }
@@ -5094,10 +5109,7 @@ int dp_mlp_train(dp_mlp* m, int64_t steps, int batch, float lr0, float lr1, floa
                  float* losses) {
     if (!m || !m->s) return fail(DP_ERR_ARG, "no training data");
     if (steps < 1 || batch < 16) return fail(DP_ERR_ARG, "bad steps / batch");
-    if (steps > m->losses_cap) {
-        RET(dalloc_t(&m->losses, (size_t)steps));
-        m->losses_cap = steps;
-    }
+    RET(dgrow_t(&m->losses, (long long)steps, &m->losses_cap));
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     MlpTrainArgs ga = mlp_grad_args(m, m->s, m->t, batch, wf);
     ga.draw = 1;
