@@ -4239,7 +4239,8 @@ int dp_time_kernel(dp_sim* s, int which, int reps, float* ms) {
             case DP_KERNEL_SKIN: return launch_skin_check(s);
             case DP_KERNEL_STEP:
                 if (!use_fused_step(s)) return fail(DP_ERR_ARG, "no fused step kernel in this mode");
-                return launch_step(s, DP_INT_GJF, 0, nullptr);
+                // as run() launches it (`far` stays as it is: the positions are not advanced)
+                return launch_step(s, DP_INT_GJF, 0, nullptr, use_own_lists(s) ? DP_END_OWN_LISTS : 0);
             default: return fail(DP_ERR_ARG, "unknown kernel");
         }
     };

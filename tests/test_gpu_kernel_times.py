@@ -44,3 +44,27 @@ def test_forces_cost_less_than_a_step(precision):
     sim = _liquid((1000, 1000), precision)
     sim.run(5)
     assert _time(sim, _lib.DP_KERNEL_FORCES) <= _time(sim, _lib.DP_KERNEL_STEP)
+
+
+@pytest.mark.parametrize("cells", [(5, 5, 5), (8, 8, 8)])
+def test_small_system_step_is_the_one_that_runs(cells):
+    """Up to 8,192 particles a run's steps rebuild their own lists; a step without a
+    rebuild costs less than the mean step of a run, and more than a third of it."""
+    from dompap_gb300 import Simulation, _lib
+    from dompap_gb300.positions import FCC
+
+    np.random.seed(1)
+    sim = Simulation()
+    sim.set_positions(unit_cell_coordinates=FCC, cells=cells, lattice_constants=(1.0, 1.0, 1.0))
+    sim.set_masses(masses=1.0)
+    sim.set_density(density=0.8442)
+    sim.set_random_velocities(temperature=1.0)
+    sim.set_pair_potential(pair_potential_str="4*(r**-12-r**-6)", r_cut=2.5)
+    sim.set_neighbor_list(skin=0.5, max_number_of_neighbors=192)
+    sim.set_integrator(time_step=0.005, target_temperature=1.0, temperature_damping_time=0.1)
+    sim.run(200)
+    before = np.array(sim.positions), sim._stats().steps
+    step = _time(sim, _lib.DP_KERNEL_STEP, 50)
+    assert np.array_equal(np.array(sim.positions), before[0]) and sim._stats().steps == before[1]
+    mean = min(sim.run_timed(1000) for _ in range(3)) / 1000
+    assert mean / 3 <= step <= mean
