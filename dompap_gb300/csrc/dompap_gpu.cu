@@ -1766,11 +1766,14 @@ static int compile_pair_lib(const std::string& src, PairLib* out) {
         CK(cudaLibraryGetKernel(&pl.step, pl.lib, "dp_step"));
         CK(cudaLibraryGetKernel(&pl.step_warp, pl.lib, "dp_step_warp"));
         CK(cudaLibraryGetKernel(&pl.step_quad, pl.lib, "dp_step_quad"));
-        CK(cudaLibraryGetKernel(&pl.step_lists, pl.lib, "dp_step_lists"));
+        if (src.find("#define DP_LISTS_BLOCKS 0\n") == std::string::npos)
+            CK(cudaLibraryGetKernel(&pl.step_lists, pl.lib, "dp_step_lists"));
         const char* quantity[4] = {"dp_forces_", "dp_energy_", "dp_virial_", "dp_laplacian_"};
-        for (int q = 0; q < 4; ++q) {
-            CK(cudaLibraryGetKernel(&pl.split[0][q], pl.lib, (std::string(quantity[q]) + "warp").c_str()));
-            CK(cudaLibraryGetKernel(&pl.split[1][q], pl.lib, (std::string(quantity[q]) + "quad").c_str()));
+        const char* lanes[2] = {"warp", "quad"};
+        for (int w = 0; w < 2; ++w) {
+            if (src.find(w == 0 ? "#define DP_WARP_SUMS 0\n" : "#define DP_QUAD_SUMS 0\n") != std::string::npos) continue;
+            for (int q = 0; q < 4; ++q)
+                CK(cudaLibraryGetKernel(&pl.split[w][q], pl.lib, (std::string(quantity[q]) + lanes[w]).c_str()));
         }
         CK(cudaLibraryGetKernel(&pl.step_all, pl.lib, "dp_step_all"));
         CK(cudaLibraryGetKernel(&pl.forces_all, pl.lib, "dp_forces_all"));
@@ -3757,11 +3760,21 @@ static std::string called_pair_functions(std::string src) {
     return src;
 }
 
+// The kernels a program has besides those of any size, and the CTAs per SM that the
+// steps are compiled for (0: without that kernel). A program with all of them takes
+// NVRTC twice as long as the part a system of one size uses (Lennard-Jones 3.9 s against
+// 1.9, the costly test potential with 32 more terms 42.7 against 9).
+struct ProgramParts {
+    int step_blocks = 6, brick_blocks = 4, lists_blocks = 4;
+    bool warp_sums = true, quad_sums = true;
+};
+
 static std::string pair_program(int dim, int precision, int pmode, bool sig_one, bool eps_one,
-                                const std::string& pot_src, bool with_batch, int step_blocks_hint = 6,
-                                int brick_blocks = 4, int lists_blocks = 4) {
+                                const std::string& pot_src, bool with_batch, const ProgramParts& parts) {
     std::string src;
-    src += "#define DP_LISTS_BLOCKS " + std::to_string(lists_blocks) + "\n";
+    src += "#define DP_LISTS_BLOCKS " + std::to_string(parts.lists_blocks) + "\n";
+    src += std::string("#define DP_WARP_SUMS ") + (parts.warp_sums ? "1" : "0") + "\n";
+    src += std::string("#define DP_QUAD_SUMS ") + (parts.quad_sums ? "1" : "0") + "\n";
     src += "#define DP_DIM " + std::to_string(dim) + "\n";
     if (precision == DP_PREC_MLP) src += "#define DP_MLP 1\n";
     if (precision == DP_PREC_FP64) src += "#define DP_FF 1\n";
@@ -3775,7 +3788,7 @@ static std::string pair_program(int dim, int precision, int pmode, bool sig_one,
     src += std::string("#define DP_EPS_ONE ") + (eps_one ? "1" : "0") + "\n";
     // resident 256-thread CTAs per SM the fused step kernel is compiled for
     // (register cap 65536 / (256 n)); DOMPAP_STEP_MIN_BLOCKS overrides
-    int step_blocks = step_blocks_hint;
+    int step_blocks = parts.step_blocks;
     if (const char* env = std::getenv("DOMPAP_STEP_MIN_BLOCKS")) step_blocks = std::atoi(env);
     src += "#define DP_STEP_MIN_BLOCKS " + std::to_string(std::max(0, std::min(8, step_blocks))) + "\n";
     src += dp_src_common;
@@ -3787,8 +3800,8 @@ static std::string pair_program(int dim, int precision, int pmode, bool sig_one,
     src += precision == DP_PREC_FP32 && pair_cost(pot_src) >= kCostlyPair ? called_pair_functions(pot_src) : pot_src;
     src += "\n// ---- pair kernels ----\n";
     src += dp_src_pair;
-    if (brick_program(dim, precision, pmode, pot_src) && !with_batch) {
-        src += "\n#define DP_BRICKS 1\n#define DP_BRICK_BLOCKS " + std::to_string(brick_blocks) + "\n";
+    if (parts.brick_blocks > 0 && brick_program(dim, precision, pmode, pot_src)) {
+        src += "\n#define DP_BRICKS 1\n#define DP_BRICK_BLOCKS " + std::to_string(parts.brick_blocks) + "\n";
         src += dp_src_brick;
     }
     if (with_batch) {
@@ -3827,12 +3840,17 @@ static int lists_blocks_for(long long n) { return n < 3072 ? 2 : 4; }
 static int rebuild_pair_lib(dp_sim* s) {
     const bool sig_one = s->pmode == DP_PAIR_CONST && s->sigma == 1.0;
     const bool eps_one = s->pmode == DP_PAIR_CONST && s->epsilon == 1.0;
-    const int step_blocks =
-        s->step_blocks ? s->step_blocks : step_blocks_for(s->dim, s->precision, s->pmode, pair_cost(s->pot_src));
+    // by the sizes at which sum_lanes, list_kind and step_lanes choose them
+    const bool small = s->n <= s->warp_step_max;
+    ProgramParts parts;
+    parts.step_blocks = s->step_blocks ? s->step_blocks
+                                       : step_blocks_for(s->dim, s->precision, s->pmode, pair_cost(s->pot_src));
+    parts.brick_blocks = small ? 0 : (s->step_blocks ? s->step_blocks : brick_blocks_for(s->n));
+    parts.lists_blocks = !small ? 0 : (s->step_blocks ? s->step_blocks : lists_blocks_for(s->n));
+    parts.warp_sums = small;
+    parts.quad_sums = !small && s->n <= s->quad_step_max;
     const std::string src =
-        pair_program(s->dim, s->precision, s->pmode, sig_one, eps_one, s->pot_src, false, step_blocks,
-                     s->step_blocks ? s->step_blocks : brick_blocks_for(s->n),
-                     s->step_blocks ? s->step_blocks : lists_blocks_for(s->n));
+        pair_program(s->dim, s->precision, s->pmode, sig_one, eps_one, s->pot_src, false, parts);
     PairLib pl;
     RET(compile_pair_lib(src, &pl));
     s->lib = pl;
@@ -4771,7 +4789,10 @@ int dp_batch_get_state(dp_batch* b, double* positions, double* velocities, int32
 int dp_batch_set_potential(dp_batch* b, const char* device_source, double r_cut) {
     if (!b || !device_source) return fail(DP_ERR_ARG, "null argument");
     if (!(r_cut > 0.0) || !std::isfinite(r_cut)) return fail(DP_ERR_ARG, "r_cut must be positive and finite");
-    const std::string src = pair_program(b->dim, DP_PREC_FP32, DP_PAIR_CONST, true, true, device_source, true);
+    ProgramParts parts;
+    parts.brick_blocks = parts.lists_blocks = 0;
+    parts.warp_sums = parts.quad_sums = false;
+    const std::string src = pair_program(b->dim, DP_PREC_FP32, DP_PAIR_CONST, true, true, device_source, true, parts);
     PairLib pl;
     RET(compile_pair_lib(src, &pl));
     if (!pl.batch[0]) return fail(DP_ERR_NVRTC, "batch kernels missing from the compiled program");
@@ -4895,8 +4916,10 @@ static int nvrtc_check_impl(int dim, int precision, int pair_mode, int with_batc
         return fail(DP_ERR_ARG, "unknown precision");
     if (pair_mode < DP_PAIR_CONST || pair_mode > DP_PAIR_DENSE) return fail(DP_ERR_ARG, "unknown pair mode");
     const bool one = pair_mode == DP_PAIR_CONST;
-    const std::string src = pair_program(dim, precision, pair_mode, one, one, device_source, with_batch != 0,
-                                         step_blocks_for(dim, precision, pair_mode, pair_cost(device_source)));
+    ProgramParts parts;  // all of them
+    parts.step_blocks = step_blocks_for(dim, precision, pair_mode, pair_cost(device_source));
+    if (with_batch) parts.brick_blocks = 0;
+    const std::string src = pair_program(dim, precision, pair_mode, one, one, device_source, with_batch != 0, parts);
     std::vector<char> cubin;
     RET(nvrtc_cubin(src, &cubin, resource_log, true, true));
     if (cubin_bytes) *cubin_bytes = (int64_t)cubin.size();

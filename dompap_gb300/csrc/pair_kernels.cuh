@@ -17,8 +17,9 @@
 // with s = r / sigma and every term 0 where s > r_cut (dompap/potential.py:61-65).
 // There is no 1/sigma chain-rule factor, exactly as in the reference.
 //
-// Layout in HBM: positions are SoA float64 pos[k*N + i]; the neighbour list
-// is column-major nl[k*N + i] with per-particle counts cnt[i]; the
+// Layout in HBM: positions are SoA float64 pos[k*N + i]; entry k of slot i's
+// neighbour list is nl[k nl_k + i nl_i] (column-major, or a row per slot where a
+// warp shares a particle) with per-particle counts cnt[i]; the
 // fixed-point shadow is one 8- or 16-byte vector per particle.
 //
 // Configuration macros (set by the host):
@@ -31,8 +32,21 @@
 //                   (dp_ff.cuh) on the exact 64-bit fixed-point displacement; the
 //                   cut decision within float rounding of r_cut and positions not
 //                   yet wrapped into the box take the float64 path
+//   DP_LISTS_BLOCKS, DP_WARP_SUMS, DP_QUAD_SUMS
+//                   kernels for sizes that the program may leave out (0): the step that
+//                   keeps its own lists (else its CTAs per SM), sums with 32 and with 4
+//                   lanes per particle
 #ifndef DP_FF
 #define DP_FF 0
+#endif
+#ifndef DP_LISTS_BLOCKS
+#define DP_LISTS_BLOCKS 4
+#endif
+#ifndef DP_WARP_SUMS
+#define DP_WARP_SUMS 1
+#endif
+#ifndef DP_QUAD_SUMS
+#define DP_QUAD_SUMS 1
 #endif
 
 #ifndef DP_DIM
@@ -670,14 +684,13 @@ extern "C" __global__ void DP_STEP_BOUNDS dp_step_quad(dp_pair_args a, dp_int_ar
 // terms, the sum over the warp, the float64 integrator) and by instruction
 // fetch. LJ, float64, a step of a run before and now: 500 particles 23.2 -> 11.9
 // us, 2,048 15.6, 4,000 60 -> 22.9, 8,112 41.
-#ifndef DP_LISTS_BLOCKS
-#define DP_LISTS_BLOCKS 4
-#endif
+#if DP_LISTS_BLOCKS > 0
 extern "C" __global__ void __launch_bounds__(256, DP_LISTS_BLOCKS) dp_step_lists(dp_pair_args a, dp_int_args b, dp_list_args l) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     dp_step_split<32, false, true>(a, b, &l);
 }
+#endif
 
 // ---------------------------------------------------------------------------
 // No neighbour list: dompap's double-loop and vectorised methods
@@ -787,8 +800,12 @@ __device__ __forceinline__ void dp_laplacian_split(const dp_pair_args& a) {
         dp_scalar_split<DP_ACC_VIRIAL, LANES>(a);                                                                   \
     }                                                                                                               \
     extern "C" __global__ void DP_FORCES_BOUNDS dp_laplacian_##NAME(dp_pair_args a) { dp_laplacian_split<LANES>(a); }
+#if DP_WARP_SUMS
 DP_SPLIT_KERNELS(warp, 32)
+#endif
+#if DP_QUAD_SUMS
 DP_SPLIT_KERNELS(quad, 4)
+#endif
 #endif
 
 // Per-block partial sums of a scalar pair quantity (energy or virial); the
